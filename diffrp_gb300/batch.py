@@ -60,6 +60,9 @@ def _register():
                                  ctypes.c_uint, P, P, P, P, LL, P, ctypes.c_float, P, P, P, P],
         "drp_batch_forward_l1_grad": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL,
                                       ctypes.c_uint, P, P, P, P, LL, P, ctypes.c_float, P, P, P, P, P, LL, P],
+        "drp_batch_fit_l1": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL,
+                             ctypes.c_uint, P, P, P, P, LL, P, ctypes.c_float, P, P, P, P, P, LL, P],
+        "drp_batch_colors": [P, I, P, LL, P, P, P, P, P],
         "drp_scale_floats": [P, P, LL, P, P],
         "drp_batch_backward": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, P, P, P, LL, P, P, P, P,
                                P, I, P],
@@ -298,9 +301,10 @@ class BatchRenderer:
         (target, scale, grad, block_loss, loss) fuses the L1 loss into the
         antialias pass (drp_batch_forward_l1); l1 = (target, scale,
         block_loss, loss, grad_pos, grad_attr) also forms the loss's gradient
-        there (drp_batch_forward_l1_grad, flags required; grad_attr and
+        there (drp_batch_fit_l1, flags required; grad_attr and
         grad_pos are accumulated, after the call zeroes the buffer given
-        last, when it is not None).  flags: an
+        last, when it is not None; color is scratch then, written only at
+        the pixels a blending pair touches).  flags: an
         antialias state block (_flags()) the forward fills for its backward,
         or None."""
         if not torch.cuda.is_current_stream_capturing():
@@ -328,7 +332,7 @@ class BatchRenderer:
             tail = (target.data_ptr(), ctypes.c_float(scale), block_loss.data_ptr(), loss.data_ptr(),
                     gpos.data_ptr(), gattr.data_ptr(), None if zero is None else zero.data_ptr(),
                     0 if zero is None else zero.numel(), stream)
-            entry = "drp_batch_forward_l1_grad"
+            entry = "drp_batch_fit_l1"
         elif l1 is not None:
             target, scale, grad, block_loss, loss = l1
             tail = (target.data_ptr(), ctypes.c_float(scale), grad.data_ptr(), block_loss.data_ptr(),
@@ -405,7 +409,7 @@ class BatchRenderer:
 
         grads_in_forward=True (items of at most 32 channels): the forward
         also forms d loss / d pos and d loss / d attr, in the pass that forms
-        the loss (drp_batch_forward_l1_grad), so that a backward reaching only
+        the loss (drp_batch_fit_l1), so that a backward reaching only
         the loss is one multiplication by its upstream gradient -- and, with
         recompute, re-renders nothing.  A backward that also reaches the
         images runs the full backward instead (the gradients formed in the
@@ -617,8 +621,12 @@ class _BatchL1GradFn(torch.autograd.Function):
                                  cr._fwd_gen, aa_flags=flags)
             return grad_pos, grad_attr, None, None
         _, rast, color = saved[5:]
-        # the gradient-forming forward fills only the state's pixel list, not
-        # its per-pixel flags: the backward evaluates every pixel's
-        # antialias terms itself
+        # the gradient-forming forward keeps no colour image (its color buffer
+        # is scratch) and fills only the state's pixel list, not its per-pixel
+        # flags: the colours are interpolated again, and the backward
+        # evaluates every pixel's antialias terms itself
+        color = torch.empty_like(color)
+        _ffi.call("drp_batch_colors", r._items_dev.data_ptr(), len(r.items), r._xmap.data_ptr(), r.pixel_blocks,
+                  r.tri.data_ptr(), attr.data_ptr(), rast.data_ptr(), color.data_ptr(), _ffi.stream_of(pos.device))
         r._backward_raw(pos, attr, rast, color, gout, grad_pos, grad_attr, ctx.gen)
         return grad_pos, grad_attr, None, None

@@ -72,24 +72,12 @@ struct AAPair {
     float2 cF, cO;
 };
 
-// Pair (A, B) with A the left / lower pixel at column ax, row ay and B its
-// right (vertical = false) or upper (vertical = true) neighbour; rA, rB their
-// rast rows; rec the view's triangle records (F triangles).
-__device__ __forceinline__ void aa_pair(const float4* rec, long long F, int A, int Bp, int ax, int ay, bool vertical,
-                                        const float4& rA, const float4& rB, AAPair& R) {
+// The part of aa_pair after the front pixel is known: its triangle T's exit
+// edge on the segment to the other pixel.
+__device__ __forceinline__ void aa_pair_edges(const float4* rec, int T, bool front_a, int A, int Bp, int ax, int ay,
+                                              bool vertical, AAPair& R) {
     R.valid = false;
-    const int tA = rast_tri(rA.w), tB = rast_tri(rB.w);
-    const int cA = (tA >= 0 && tA < F) ? tA : -1;
-    const int cB = (tB >= 0 && tB < F) ? tB : -1;
-    if (cA == cB) return;
-    int Fp;
-    if (cA < 0) Fp = Bp;
-    else if (cB < 0) Fp = A;
-    else if (rA.z < rB.z) Fp = A;
-    else if (rB.z < rA.z) Fp = Bp;
-    else Fp = cA < cB ? A : Bp;
-    const int Op = (Fp == A) ? Bp : A;
-    const int T = (Fp == A) ? cA : cB;
+    const int Fp = front_a ? A : Bp, Op = front_a ? Bp : A;
     const float4 q1 = rec[2 * (long long)T + 1];
     const float sgn = q1.z;
     const unsigned mask = __float_as_uint(q1.w);
@@ -104,8 +92,8 @@ __device__ __forceinline__ void aa_pair(const float4* rec, long long F, int A, i
     const float2 ctrA = make_float2((float)ax + 0.5f, (float)ay + 0.5f);
     const float2 ctrB = vertical ? make_float2(ctrA.x, (float)(ay + 1) + 0.5f)
                                  : make_float2((float)(ax + 1) + 0.5f, ctrA.y);
-    R.cF = Fp == A ? ctrA : ctrB;
-    R.cO = Fp == A ? ctrB : ctrA;
+    R.cF = front_a ? ctrA : ctrB;
+    R.cO = front_a ? ctrB : ctrA;
     int best = -1;
     float bt = 0.f, beF = 0.f, beO = 0.f;
 #pragma unroll
@@ -143,6 +131,25 @@ __device__ __forceinline__ void aa_pair(const float4* rec, long long F, int A, i
         R.sign = -1.0f;
     }
     R.valid = true;
+}
+
+// Pair (A, B) with A the left / lower pixel at column ax, row ay and B its
+// right (vertical = false) or upper (vertical = true) neighbour; rA, rB their
+// rast rows; rec the view's triangle records (F triangles).
+__device__ __forceinline__ void aa_pair(const float4* rec, long long F, int A, int Bp, int ax, int ay, bool vertical,
+                                        const float4& rA, const float4& rB, AAPair& R) {
+    R.valid = false;
+    const int tA = rast_tri(rA.w), tB = rast_tri(rB.w);
+    const int cA = (tA >= 0 && tA < F) ? tA : -1;
+    const int cB = (tB >= 0 && tB < F) ? tB : -1;
+    if (cA == cB) return;
+    int Fp;
+    if (cA < 0) Fp = Bp;
+    else if (cB < 0) Fp = A;
+    else if (rA.z < rB.z) Fp = A;
+    else if (rB.z < rA.z) Fp = Bp;
+    else Fp = cA < cB ? A : Bp;
+    aa_pair_edges(rec, Fp == A ? cA : cB, Fp == A, A, Bp, ax, ay, vertical, R);
 }
 
 // Pair slot q of a pixel, in the fixed order left, right, below, above:
@@ -275,6 +282,17 @@ __device__ __forceinline__ bool aa_fwd_terms_row(const float4* R, const float4* 
     }
     if (pair_bits) *pair_bits = bits;
     return any;
+}
+
+// A pixel's word as the batched fine raster writes it: its triangle + 1 (0:
+// background) and kPixSil when that triangle's antialias record has a
+// silhouette edge.  A pair whose front triangle has none never blends
+// (aa_pair), so two unequal ids without the bit need no record and no rast
+// row: inside a closed mesh that is almost every pair.
+constexpr uint32_t kPixSil = 0x80000000u;
+
+__device__ __forceinline__ bool pix_pair_may_blend(uint32_t a, uint32_t b) {
+    return ((a ^ b) & ~kPixSil) != 0u && ((a | b) & kPixSil) != 0u;
 }
 
 // Forward of one pixel: out = c + sum over pair slots targeting this pixel of

@@ -49,6 +49,9 @@ struct BatchArgs {
     unsigned char* aa_flags;
     int* aa_list;
     unsigned* aa_count;
+    bool fit;               // the gradient-forming loss pass is batch_fit_kernel
+    uint32_t* aa_words;     // per pixel: triangle + 1 (0: none), kPixSil where its record has a silhouette edge
+    bool emit_color;        // fit: the fine raster writes the colour of every pixel
     bool emit_out;          // the fine raster also writes the colour into out
     bool aa_records;        // the setup pass writes the antialias triangle records
     // fused mean-absolute-error loss (null target: none)
@@ -67,6 +70,7 @@ struct BatchArgs {
     // workspace
     uint32_t* stats;
     uint32_t* queue;
+    uint32_t* loss_count;  // CTAs of the list kernel that have added their slice of the loss
     int4* prims;
     uint32_t *tile_count, *tile_offset, *tile_cursor, *tile_list;
     unsigned long long* chunk_sums;  // tile-scan chunk sums
@@ -149,6 +153,7 @@ __global__ void __launch_bounds__(2 * kSetupTris) batch_setup_bin_kernel(BatchAr
 // rast + interpolated attributes of one pixel (interpolator.py:45 order).
 // The colour also goes to out (when not null): the antialias pass then only
 // rewrites the pixels it blends.
+template <bool FIT>
 struct BatchEmit {
     const float4* P;
     const int* tri;  // the item's mesh triangles (local vertex indices)
@@ -156,14 +161,20 @@ struct BatchEmit {
     int W, H, C;
     bool vec;  // 128-bit attribute / colour / output access: C % 4 == 0 and all bases 16-byte aligned
     float4* rast;
-    float* color;
+    float* color;       // FIT: null where only the listed pixels' colours are wanted
     float* out;
+    uint32_t* words;    // FIT: the item's pixel words
+    const float4* rec;  // FIT: the item's antialias records
     __device__ __forceinline__ void operator()(int px, int py, unsigned long long k, float X, float Y) const {
         const long long o = (long long)py * W + px;
         float* col = color + o * C;
         float* oc = out ? out + o * C : nullptr;
         if (k == ~0ull) {
             rast[o] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (FIT) {
+                words[o] = 0u;
+                if (!color) return;
+            }
             if (vec) {
                 for (int c = 0; c < C; c += 4) {
                     *reinterpret_cast<float4*>(col + c) = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -182,6 +193,10 @@ struct BatchEmit {
         Shade S;
         shade_eval_xy(P[i0], P[i1], P[i2], X, Y, W, H, S);
         rast[o] = make_float4(S.u, S.v, S.zw, enc_triid(t + 1));
+        if (FIT) {
+            words[o] = (uint32_t)(t + 1) | (__float_as_uint(rec[2 * (long long)t + 1].w) ? kPixSil : 0u);
+            if (!color) return;
+        }
         const float* a0 = A + (long long)i0 * C;
         const float* a1 = A + (long long)i1 * C;
         const float* a2 = A + (long long)i2 * C;
@@ -218,7 +233,7 @@ __device__ __forceinline__ int find_item_by_tile(const drp_batch_item* items, in
     return lo;
 }
 
-template <int TILE_LOG2, int TPT>
+template <int TILE_LOG2, int TPT, bool FIT>
 __global__ void __launch_bounds__((1 << (2 * TILE_LOG2)) < 256 ? (1 << (2 * TILE_LOG2)) : 256,
                                   TILE_LOG2 == 3 ? 12 : 4)
 batch_fine_kernel(BatchArgs a) {
@@ -227,7 +242,7 @@ batch_fine_kernel(BatchArgs a) {
     // working set past the 64 registers of 4 CTAs per SM (spills).
     __shared__ long long job;
     __shared__ FineTile ft;
-    __shared__ BatchEmit e;
+    __shared__ BatchEmit<FIT> e;
     pdl_wait();
     pdl_launch_dependents();
     for (;;) {
@@ -268,8 +283,12 @@ batch_fine_kernel(BatchArgs a) {
                 e.H = it.height;
                 e.C = it.channels;
                 e.rast = reinterpret_cast<float4*>(a.rast) + it.pixel_offset;
-                e.color = a.color + it.image_offset;
+                e.color = !FIT || a.emit_color ? a.color + it.image_offset : nullptr;
                 e.out = a.emit_out ? a.out + it.image_offset : nullptr;
+                if (FIT) {
+                    e.words = a.aa_words + it.pixel_offset;
+                    e.rec = a.aa_rec + it.prim_offset * 2;
+                }
                 e.vec = (it.channels & 3) == 0 &&
                         ((reinterpret_cast<uintptr_t>(e.A) | reinterpret_cast<uintptr_t>(e.color) |
                           reinterpret_cast<uintptr_t>(e.out)) & 15) == 0;
@@ -414,6 +433,54 @@ struct ItemGrad<true> {
     }
 };
 
+// Launches of at least this many pixels form the loss and its gradient with
+// batch_fit_kernel, smaller ones with batch_aa_l1_grad_kernel, whose shorter
+// chain per pixel is what counts while the regions fill only part of the chip:
+// one view of 400 x 400 takes 58.5 with the first against 55.3 us per step with
+// the second at 3 channels and 68.2 against 63.8 at 8; 724 x 724 84.2 against
+// 88.6 and 81.2 against 84.0 (but 12 channels 6 percent more); from 1024 x 1024
+// on 3 to 8 and 16 channels are 7 to 40 percent faster, 12 even.
+constexpr long long kFitPixels = 1ll << 20;
+
+// batch_fit_kernel takes regions of 32 x 16 pixels, a fixed number per raster
+// tile in grid order: the halves of a 32-pixel tile, a pair of 16-pixel tiles
+// or a 4 x 2 block of 8-pixel ones (their first tile takes it, the others
+// nothing).  Region i leaves its |error| sum in a tile word the raster has
+// spent: the tile's list offset, or for the second half its cursor.
+__host__ __device__ inline int fit_regions_per_tile(int tile_log2) { return tile_log2 == 5 ? 2 : 1; }
+
+__device__ __forceinline__ float* fit_loss_slot(const BatchArgs& a, long long i) {
+    if (a.tile_log2 != 5) return reinterpret_cast<float*>(a.tile_offset + i);
+    return reinterpret_cast<float*>(((i & 1) ? a.tile_cursor : a.tile_offset) + (i >> 1));
+}
+
+// The loss from the regions' sums: every CTA adds a contiguous slice of them
+// and leaves its sum in the slice's first slot; the CTA that arrives last (a
+// counter the forward's first kernel zeroed; nobody waits) adds the slices.
+// Fixed slices, fixed order within each: reproducible.  One CTA adding every
+// partial took 27 us of the 64-view step.
+__device__ __forceinline__ void fit_loss(const BatchArgs& a) {
+    __shared__ float total;
+    __shared__ bool last;
+    const long long n = a.total_tiles * fit_regions_per_tile(a.tile_log2);
+    const long long per = (n + gridDim.x - 1) / gridDim.x;
+    const long long b0 = blockIdx.x * per, b1 = b0 + per < n ? b0 + per : n;
+    float s = 0.f, c = 0.f;
+    for (long long i = b0 + threadIdx.x; i < b1; i += blockDim.x) two_sum(s, c, *fit_loss_slot(a, i));
+    block_sum_pairs<kFinalThreads>(s, c, 1.0f, &total);
+    if (threadIdx.x == 0) {
+        if (b0 < b1) *fit_loss_slot(a, b0) = total;
+        __threadfence();
+        last = atomicAdd(a.loss_count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    s = c = 0.f;
+    for (long long b = threadIdx.x * per; b < n; b += blockDim.x * per) two_sum(s, c, __ldcg(fit_loss_slot(a, b)));
+    block_sum_pairs<kFinalThreads>(s, c, a.l1_scale, a.loss);
+}
+
 // Lanes per listed pixel in batch_aa_bwd_kernel.  Two lanes cover twice the
 // pixels of four per resident wave (the single-mesh step lists ~45K pixels:
 // one wave with two, two with four), but each lane's chain of slot
@@ -424,16 +491,23 @@ struct ItemGrad<true> {
 #endif
 constexpr int kListLanes = DRP_LIST_LANES;
 
-template <bool L1G, int LANES>
+// Who launches it: the ordinary backward, or the forward that forms the loss's
+// gradient, after batch_aa_l1_grad_kernel or batch_fit_kernel.  (The two sums
+// of the loss are separate instantiations: with both in one the list of small
+// launches took 16.5 instead of 15.8 us, one view of 256 x 256 x 3.)
+constexpr int kListBackward = 0, kListL1 = 1, kListFit = 2;
+
+template <int KIND, int LANES>
 __global__ void __launch_bounds__(256) batch_aa_bwd_kernel(BatchArgs a) {
+    constexpr bool L1G = KIND != kListBackward;
     static_assert(LANES == 2 || LANES == 4, "two or four lanes per listed pixel");
     constexpr int SLOTS = 4 / LANES;  // pair slots each lane evaluates
     pdl_wait();
     pdl_launch_dependents();
-    // the forward that forms the loss's gradient ends here: its last block
-    // also adds the loss (the partials of the antialias / loss pass)
     static_assert(kFinalThreads == 256, "the list kernel's blocks form the loss");
-    if (L1G && blockIdx.x == gridDim.x - 1)
+    if (KIND == kListFit)
+        fit_loss(a);
+    else if (KIND == kListL1 && blockIdx.x == gridDim.x - 1)
         l1_final_block<kFinalThreads>(a.block_loss, a.n_pix_blocks, a.l1_scale, a.loss);
     const unsigned n = *a.aa_count;
     const float gsc = (!L1G && a.grad_scale) ? *a.grad_scale : 1.0f;
@@ -542,12 +616,12 @@ __global__ void __launch_bounds__(256) batch_aa_bwd_kernel(BatchArgs a) {
 
 // One resident wave of the listed-pixel kernel (its CTAs per SM from the
 // occupancy query, cached per instantiation), capped by the pixel blocks.
-template <bool L1G>
+template <int KIND>
 static long long list_kernel_grid(long long pix_blocks) {
     static std::atomic<int> per_sm{0};
     int per = per_sm.load(std::memory_order_relaxed);
     if (per == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_aa_bwd_kernel<L1G, kListLanes>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_aa_bwd_kernel<KIND, kListLanes>, 256, 0);
         per = per > 0 ? per : 1;
         per_sm.store(per, std::memory_order_relaxed);
     }
@@ -688,6 +762,702 @@ __global__ void __launch_bounds__(256, 4) batch_bwd_kernel(BatchArgs a) {
     }
 }
 
+// Interpolated channels [c0, c0 + 4) of a pixel from its rast row and vertex
+// indices (t < 0: background), as BatchEmit writes them; channels past C are 0.
+// x0..x2 get the three vertices' values (0 for background).  VEC: C % 4 == 0
+// and 16-byte aligned attributes.
+template <bool VEC>
+__device__ __forceinline__ void lerp_group(const float* A, int C, int c0, int t, int i0, int i1, int i2, float u,
+                                           float v, float (&x0)[4], float (&x1)[4], float (&x2)[4], float (&col)[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x0[k] = x1[k] = x2[k] = col[k] = 0.f;
+    if (t < 0) return;
+    if (VEC) {
+        const float4 q0 = __ldg(reinterpret_cast<const float4*>(A + (long long)i0 * C + c0));
+        const float4 q1 = __ldg(reinterpret_cast<const float4*>(A + (long long)i1 * C + c0));
+        const float4 q2 = __ldg(reinterpret_cast<const float4*>(A + (long long)i2 * C + c0));
+        x0[0] = q0.x; x0[1] = q0.y; x0[2] = q0.z; x0[3] = q0.w;
+        x1[0] = q1.x; x1[1] = q1.y; x1[2] = q1.z; x1[3] = q1.w;
+        x2[0] = q2.x; x2[1] = q2.y; x2[2] = q2.z; x2[3] = q2.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (c0 + k < C) {
+                x0[k] = A[(long long)i0 * C + c0 + k];
+                x1[k] = A[(long long)i1 * C + c0 + k];
+                x2[k] = A[(long long)i2 * C + c0 + k];
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) col[k] = fmaf(x0[k] - x2[k], u, fmaf(x1[k] - x2[k], v, x2[k]));
+}
+
+// l1_sign in three instructions (setp.ne is false for NaN, as both compares are).
+__device__ __forceinline__ float l1_sign_fast(float d, float scale) {
+    float g;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.f32 p, %1, 0f00000000;\n\tselp.f32 %0, %2, 0f00000000, p;\n\t}"
+        : "=f"(g)
+        : "f"(d), "f"(__uint_as_float((__float_as_uint(d) & 0x80000000u) ^ __float_as_uint(scale))));
+    return g;
+}
+
+// Four channels of an image row: one vector (VEC) or the channels below C.
+template <bool VEC>
+__device__ __forceinline__ void load4(const float* p, int n, float (&x)[4]) {
+    if (VEC) {
+        const float4 q = *reinterpret_cast<const float4*>(p);
+        x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = k < n ? p[k] : 0.f;
+    }
+}
+
+template <bool VEC>
+__device__ __forceinline__ void store4(float* p, int n, const float (&x)[4]) {
+    if (VEC) {
+        *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < n) p[k] = x[k];
+    }
+}
+
+// Antialias + L1 loss with the loss's gradient formed in the same pass, for
+// launches of at least kFitPixels (drp_batch_fit_l1,
+// drp_batch_forward_l1_grad).  Every pixel: its colour, interpolated again
+// from its rast row (the attribute rows are needed for the backward anyway, so
+// no colour image is written and read back), the blend, the output and the
+// |error| sum.  Then, for the pixels no blending pair touches (the listed ones
+// belong to batch_aa_bwd_kernel, which forms the sign from the output
+// and the target), the pixel's whole backward with g = sign(out - target) *
+// scale, as batch_aa_l1_grad_kernel forms it.
+//
+// A warp first finds the pairs that may blend and evaluates them together
+// (fit_pairs), then walks its rows down, one column per lane, and keeps the
+// sums of the triangle its column is in as registers (eight channels x three
+// vertices and the three positions): a triangle several pixels tall costs one
+// fused multiply-add per value and pixel, and a row of floats in shared memory
+// only where a column leaves it.  32 such rows are then added by columns and
+// go out with one vector atomic per run of rows of one triangle (fit_drain).
+// Rast rows and target come by asynchronous copies two rows ahead.
+//
+// What bounds it: issue and the latency of the gathers at 16 warps per SM.
+// One thread per pixel with segmented shuffles took 1270 warp instructions
+// per 32 pixels on 64 views of 512 x 512 x 8 channels, most of them predicated
+// shuffle steps and pair evaluation for a lane or two at a time; this takes
+// about 500, and the pass
+// 516 instead of 951 us (step 937 instead of 1414); on one 1024 x 1024 view 65
+// instead of 77 us (127 instead of 137).
+// Floats per shared row: 24 attribute sums (per four channels three vertices),
+// three position sums (x, y, 0, w), the vertex indices; eight lanes' float4
+// stores cover the banks.
+constexpr int kFitRow = 44;
+constexpr int kFitStages = 3;  // rows of a walk in flight or in use
+
+// One warp's shared memory: the pair terms first, then the walk.
+struct FitPairsShared {
+    uint32_t words[10][36];       // the rows' words with one pixel around them (column 1 + lane)
+    unsigned short queue[8 * 72];  // pairs to evaluate: lane | row << 5 | slot << 8
+    float wt[8][32][4];           // weight of a pixel's slot
+    uint32_t flags[8][32];        // slots that blend | slots that blend into the pixel << 4
+    unsigned short blend[256];    // blended pixels: lane | row << 5
+};
+struct FitWalkShared {
+    float rows[32][kFitRow];
+    float4 rast[kFitStages][32];       // the walk's rows: rast and
+    float4 target[kFitStages][2][32];  // target (groups of four channels)
+};
+union FitShared {
+    FitPairsShared p;
+    FitWalkShared w;
+};
+
+// Adds the first n rows of sh.rows into the gradients: NG groups of four
+// channels from c0 and, with POS, the clip positions.  Lane (r, q) adds quad q
+// of the r-th part of the rows; where a run of rows of one triangle (or the
+// part) ends, one vector atomic adds its four sums.
+template <int NG, bool POS, bool VEC>
+__device__ __forceinline__ void fit_drain(const BatchArgs& a, const drp_batch_item& it, FitWalkShared& sh, int n,
+                                          int c0) {
+    constexpr int Q = 3 * NG + (POS ? 3 : 0), PARTS = 32 / Q, LEN = (32 + PARTS - 1) / PARTS;
+    const int lane = threadIdx.x & 31, C = it.channels;
+    __syncwarp();
+    int4 id = make_int4(-1, -1, -1, 0);
+    if (lane < n) id = *reinterpret_cast<const int4*>(&sh.rows[lane][36]);
+    const int nx = __shfl_down_sync(0xffffffffu, id.x, 1), ny = __shfl_down_sync(0xffffffffu, id.y, 1),
+              nz = __shfl_down_sync(0xffffffffu, id.z, 1);
+    const unsigned ends = __ballot_sync(0xffffffffu, lane == 31 || nx != id.x || ny != id.y || nz != id.z);
+    const int rq = lane / Q, cq = lane - rq * Q, first = rq * LEN, len = min(n - first, LEN);
+    if (rq < PARTS && len > 0) {
+        const unsigned my_ends = (ends >> first) | (1u << (len - 1));
+        const bool attr_q = cq < 3 * NG;
+        const int slot = cq % 3, cg = c0 + 4 * (cq / 3);
+        float* base = attr_q ? a.grad_attr + it.attr_offset + cg : a.grad_pos + 4 * it.pos_offset;
+        const int stride = attr_q ? C : 4;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < LEN; ++k) {
+            if (k >= len) break;
+            const float* row = sh.rows[first + k];
+            const float4 x = *reinterpret_cast<const float4*>(row + 4 * cq);
+            acc.x += x.x;
+            acc.y += x.y;
+            acc.z += x.z;
+            acc.w += x.w;
+            if ((my_ends >> k) & 1u) {
+                float* d = base + (long long)__float_as_int(row[36 + slot]) * stride;
+                if (VEC || !attr_q) {
+                    atomic_add4(reinterpret_cast<float4*>(d), acc);
+                } else {
+                    atomicAdd(d, acc.x);
+                    if (cg + 1 < C) atomicAdd(d + 1, acc.y);
+                    if (cg + 2 < C) atomicAdd(d + 2, acc.z);
+                    if (cg + 3 < C) atomicAdd(d + 3, acc.w);
+                }
+                acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// What a pixel of the warp's rows is, one bit per row and lane: on a triangle
+// and in no blending pair (live: its backward is done here), written here (not
+// blended into), and in the list of batch_aa_bwd_kernel.
+struct FitClass {
+    unsigned live, plain, listed;
+};
+
+// Inclusive prefix sum over the warp.
+__device__ __forceinline__ int warp_prefix(int v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += y;
+    }
+    return v;
+}
+
+// Pair terms of the rows [y0, y1) (at most ROWS) x columns [x0, x0 + 32) by one
+// warp, and with them everything of the pixels a pair blends into: their
+// output and |error| (returned, per lane).  The words decide which pairs may
+// blend (the row's right neighbours and the upper ones; at the region's left
+// and lower border the outer pairs too, so a pair inside is evaluated once);
+// those go through a queue, so that 32 lanes evaluate 32 pairs -- left in
+// place, a row with one such pair would run its chain of dependent loads
+// (depths, record, edge functions) for that lane alone.  The blended pixels are
+// then done one lane per (pixel, group of four channels), and the listed ones
+// take their places in the list with one atomic.
+template <bool VEC, int ROWS>
+__device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item& it, FitPairsShared& sh, int x0,
+                                        int y0, int y1, FitClass& cl) {
+    const int lane = threadIdx.x & 31, x = x0 + lane;
+    const int W = it.width, H = it.height, C = it.channels;
+    const bool in = x < W;
+    const float4* R = reinterpret_cast<const float4*>(a.rast) + it.pixel_offset;
+    const uint32_t* Wd = a.aa_words + it.pixel_offset;
+    const int* tri = a.tri + 3 * (long long)it.tri_first;
+    const float* A = a.attr + it.attr_offset;
+    const int p0 = y0 * W + x;
+    const bool has_left = lane == 0 && x > 0, has_right = lane == 31 && x + 1 < W;
+    uint32_t w[ROWS + 2], side[ROWS];  // rows y0 - 1 .. y1
+#pragma unroll
+    for (int r = 0; r < ROWS + 2; ++r) {
+        const int y = y0 - 1 + r;
+        w[r] = in && y >= 0 && y < H && y <= y1 ? Wd[p0 + (r - 1) * W] : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+        side[r] = y0 + r < y1 && (has_left || has_right) ? Wd[p0 + r * W + (lane == 0 ? -1 : 1)] : 0u;
+    unsigned need = 0u;  // four bits per row
+    cl.live = cl.plain = cl.listed = 0u;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        uint32_t nb = __shfl_down_sync(0xffffffffu, w[r + 1], 1);
+        if (lane == 31) nb = side[r];
+        const int y = y0 + r;
+        if (!in || y >= y1) continue;
+        cl.plain |= 1u << r;
+        if (w[r + 1] & ~kPixSil) cl.live |= 1u << r;
+        if (x + 1 < W && pix_pair_may_blend(w[r + 1], nb)) need |= 2u << (4 * r);
+        if (y + 1 < H && pix_pair_may_blend(w[r + 1], w[r + 2])) need |= 8u << (4 * r);
+        if (has_left && pix_pair_may_blend(w[r + 1], side[r])) need |= 1u << (4 * r);
+        if (r == 0 && y > 0 && pix_pair_may_blend(w[1], w[0])) need |= 4u;
+    }
+    float sum = 0.f;
+    const int last = warp_prefix(__popc(need)), total = __shfl_sync(0xffffffffu, last, 31);
+    if (total) {
+        {
+            int e = last - __popc(need);
+            for (unsigned m = need; m; m &= m - 1) {
+                const int b = __ffs(m) - 1;
+                sh.queue[e++] = (unsigned short)(lane | ((b >> 2) << 5) | ((b & 3) << 8));
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS + 2; ++r) sh.words[r][1 + lane] = w[r];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            sh.flags[r][lane] = 0u;
+            if (lane == 0) sh.words[r + 1][0] = side[r];
+            if (lane == 31) sh.words[r + 1][33] = side[r];
+        }
+        __syncwarp();
+        const float4* rec = a.aa_rec + it.prim_offset * 2;
+        for (int k = lane; k < total; k += 32) {
+            const int e = sh.queue[k], l = e & 31, r = (e >> 5) & 7, q = e >> 8;
+            const int dx = q == 0 ? -1 : (q == 1 ? 1 : 0), dy = q == 2 ? -1 : (q == 3 ? 1 : 0);
+            const int px = x0 + l, py = y0 + r, pix = py * W + px;
+            const float zs = reinterpret_cast<const float*>(R + pix)[2];
+            const float zn = reinterpret_cast<const float*>(R + pix + dx + dy * W)[2];
+            const int t = (int)(sh.words[r + 1][l + 1] & ~kPixSil) - 1;
+            const int tn = (int)(sh.words[r + 1 + dy][l + 1 + dx] & ~kPixSil) - 1;
+            // the front pixel as aa_pair chooses it: the nearer one, or the
+            // only covered one; equal depths: the lower triangle
+            const bool self_front = tn < 0 || (t >= 0 && (zs < zn || (!(zn < zs) && t < tn)));
+            int A_, B_, ax, ay;
+            bool vert;
+            pair_slot(q, pix, px, py, W, H, A_, B_, ax, ay, vert);
+            AAPair pr;
+            aa_pair_edges(rec, self_front ? t : tn, self_front == (A_ == pix), A_, B_, ax, ay, vert, pr);
+            if (!pr.valid) continue;
+            const bool mine = pr.target == pix;
+            atomicOr(&sh.flags[r][l], (mine ? 17u : 1u) << q);
+            sh.wt[r][l][q] = pr.w;
+            if ((q == 1 && l < 31) || (q == 3 && py + 1 < y1)) {  // the neighbour is this warp's too: its opposite slot
+                atomicOr(&sh.flags[r + dy][l + dx], (mine ? 1u : 17u) << (q - 1));
+                sh.wt[r + dy][l + dx][q - 1] = pr.w;
+            }
+        }
+        __syncwarp();
+        unsigned blended = 0u;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            const uint32_t f = sh.flags[r][lane];
+            if (f & 15u) cl.listed |= 1u << r;
+            if (f >> 4) blended |= 1u << r;
+        }
+        cl.live &= ~cl.listed;
+        cl.plain &= ~blended;
+        // listed pixels
+        const int lend = warp_prefix(__popc(cl.listed));
+        unsigned base = 0u;
+        if (lane == 31 && lend) base = atomicAdd(a.aa_count, (unsigned)lend);
+        base = __shfl_sync(0xffffffffu, base, 31) + (unsigned)(lend - __popc(cl.listed));
+        for (unsigned m = cl.listed; m; m &= m - 1)
+            a.aa_list[base++] = (int)(it.pixel_offset + p0 + (__ffs(m) - 1) * W);
+        // blended pixels
+        const int bend = warp_prefix(__popc(blended)), nb = __shfl_sync(0xffffffffu, bend, 31);
+        {
+            int e = bend - __popc(blended);
+            for (unsigned m = blended; m; m &= m - 1) sh.blend[e++] = (unsigned short)(lane | ((__ffs(m) - 1) << 5));
+        }
+        __syncwarp();
+        const int per = (C + 3) >> 2, tasks = nb * per;
+#pragma unroll 1
+        for (int k = lane; k < tasks; k += 32) {
+            const int e = k / per, cg = 4 * (k - e * per);
+            const int l = sh.blend[e] & 31, r = sh.blend[e] >> 5;
+            const int p = (y0 + r) * W + x0 + l;
+            int slots = (int)(sh.flags[r][l] >> 4);
+            const long long prow = it.image_offset + (long long)p * C + cg;
+            float tg[4], y[3][4], base4[4], sv[4], val[4];
+            load4<VEC>(a.target + prow, C - cg, tg);
+            // the pixel and its sources in slot order (one as a rule): each
+            // source's gathers are issued beside the ones before it
+            auto vertices = [&](int sp, uint32_t word, float4& rp, int& t, int& j0, int& j1, int& j2) {
+                rp = R[sp];
+                t = (int)(word & ~kPixSil) - 1;
+                j0 = j1 = j2 = 0;
+                if (t >= 0) {
+                    j0 = tri[3 * (long long)t];
+                    j1 = tri[3 * (long long)t + 1];
+                    j2 = tri[3 * (long long)t + 2];
+                }
+            };
+            float4 rp, rs;
+            int t, j0, j1, j2, ts, k0, k1, k2;
+            vertices(p, sh.words[r + 1][l + 1], rp, t, j0, j1, j2);
+            int q = __ffs(slots) - 1;
+            auto source = [&]() {
+                const int dx = q == 0 ? -1 : (q == 1 ? 1 : 0), dy = q == 2 ? -1 : (q == 3 ? 1 : 0);
+                vertices(p + dx + dy * W, sh.words[r + 1 + dy][l + 1 + dx], rs, ts, k0, k1, k2);
+            };
+            source();
+            lerp_group<VEC>(A, C, cg, t, j0, j1, j2, rp.x, rp.y, y[0], y[1], y[2], base4);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) val[c] = base4[c];
+            for (;;) {
+                lerp_group<VEC>(A, C, cg, ts, k0, k1, k2, rs.x, rs.y, y[0], y[1], y[2], sv);
+                const float wq = sh.wt[r][l][q];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) val[c] = fmaf(wq, sv[c] - base4[c], val[c]);
+                slots &= slots - 1;
+                if (!slots) break;
+                q = __ffs(slots) - 1;
+                source();
+            }
+            store4<VEC>(a.out + prow, C - cg, val);
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (VEC || cg + c < C) sum += fabsf(val[c] - tg[c]);
+        }
+    }
+    if (C > 32) cl.live = 0u;
+    return sum;
+}
+
+// Four channels (those below n) as two pairs.
+template <bool VEC>
+__device__ __forceinline__ ulonglong2 load_pairs(const float* p, int n) {
+    if constexpr (VEC) {
+        return __ldg(reinterpret_cast<const ulonglong2*>(p));
+    } else {
+        float x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = k < n ? __ldg(p + k) : 0.f;
+        return make_ulonglong2(pack2(x[0], x[1]), pack2(x[2], x[3]));
+    }
+}
+
+// The rows [y0, y1) x columns [x0, x0 + 32) of an item of 4 NG channels with
+// 16-byte aligned rows (VEC), or of up to 4 NG channels, by one warp; returns
+// the lane's |error| sum.  Pairs of channels share instructions (fma2).
+template <int NG, bool VEC>
+__device__ __forceinline__ float fit_walk(const BatchArgs& a, const drp_batch_item& it, FitWalkShared& sh, int x0,
+                                          int y0, int y1, const FitClass& cl) {
+    const int C = VEC ? 4 * NG : it.channels;
+    const int lane = threadIdx.x & 31, x = x0 + lane;
+    const int W = it.width;
+    const bool in = x < W;
+    const float4* R = reinterpret_cast<const float4*>(a.rast) + it.pixel_offset;
+    const uint32_t* Wd = a.aa_words + it.pixel_offset;
+    const int* tri = a.tri + 3 * (long long)it.tri_first;
+    const float* A = a.attr + it.attr_offset;
+    const long long image_offset = it.image_offset;  // the stores below could alias it
+    const float4* P = reinterpret_cast<const float4*>(a.pos) + it.pos_offset;
+    const float X = fmaf((float)(2 * x + 1), __frcp_rn((float)W), -1.0f), rh = __frcp_rn((float)it.height);
+    const f32x2 minus1 = pack2(-1.0f, -1.0f);
+    float s = 0.f;
+    int n = 0;
+    // the column's triangle: sums (vertex i, channels 2 k, 2 k + 1), position sums, vertices
+    f32x2 acc[3][2 * NG];
+    float pv[9];
+    int cur = -1, j0 = 0, j1 = 0, j2 = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int k = 0; k < 2 * NG; ++k) acc[i][k] = 0ull;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) pv[k] = 0.f;
+    auto leave = [&](int e) {  // the column's sums as row e
+        f32x2* d = reinterpret_cast<f32x2*>(sh.rows[e]);
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                *reinterpret_cast<ulonglong2*>(d + 6 * g + 2 * i) = make_ulonglong2(acc[i][2 * g], acc[i][2 * g + 1]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            *reinterpret_cast<float4*>(d + 6 * NG + 2 * i) =
+                make_float4(pv[3 * i], pv[3 * i + 1], 0.f, pv[3 * i + 2]);
+        *reinterpret_cast<int4*>(d + 18) = make_int4(j0, j1, j2, 0);
+    };
+
+    // Rast rows and target arrive in shared memory two rows ahead of their use
+    // (asynchronous copies: they hold no registers), words too, vertex indices one.
+    int pix = y0 * W + x;
+    auto request = [&](int y) {
+        if (in && y < y1) {
+            const int st = (y - y0) % kFitStages, p = y * W + x;
+            cp_async<16>(&sh.rast[st][lane], R + p);
+            const float* tg = a.target + image_offset + (long long)p * C;
+#pragma unroll
+            for (int g = 0; g < NG; ++g) {
+                float* d = reinterpret_cast<float*>(&sh.target[st][g][lane]);
+                if (VEC) {
+                    cp_async<16>(d, tg + 4 * g);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (4 * g + k < C) cp_async<4>(d + k, tg + 4 * g + k);
+                }
+            }
+        }
+        cp_async_commit();
+    };
+    if (!VEC) {  // channels past the last stay zero
+#pragma unroll
+        for (int k = 0; k < kFitStages; ++k)
+#pragma unroll
+            for (int c = 0; c < 4 * NG; ++c)
+                if (c >= C) reinterpret_cast<float*>(&sh.target[k][c >> 2][lane])[c & 3] = 0.f;
+    }
+    request(y0);
+    request(y0 + 1);
+    int t = -1, t_n = -1, i0 = 0, i1 = 0, i2 = 0;
+    if (in) {
+        t = (int)(Wd[pix] & ~kPixSil) - 1;
+        if (y0 + 1 < y1) t_n = (int)(Wd[pix + W] & ~kPixSil) - 1;
+    }
+    if (t >= 0) {
+        i0 = tri[3 * (long long)t];
+        i1 = tri[3 * (long long)t + 1];
+        i2 = tri[3 * (long long)t + 2];
+    }
+    int st = 0;
+#pragma unroll 1
+    for (int yy = y0; yy < y1; ++yy) {
+        const unsigned bit = 1u << (yy - y0);
+        request(yy + 2);
+        int t_nn = -1, n0 = 0, n1 = 0, n2 = 0;
+        if (in && yy + 2 < y1) t_nn = (int)(Wd[pix + 2 * W] & ~kPixSil) - 1;
+        if (t_n >= 0) {
+            n0 = tri[3 * (long long)t_n];
+            n1 = tri[3 * (long long)t_n + 1];
+            n2 = tri[3 * (long long)t_n + 2];
+        }
+        const bool live = cl.live & bit;
+
+        // a column that enters another triangle leaves its sums behind
+        const bool enter = live && t != cur;
+        const unsigned fm = __ballot_sync(0xffffffffu, enter && cur >= 0);
+        if (fm) {
+            if (n + __popc(fm) > 32) {
+                fit_drain<NG, true, VEC>(a, it, sh, n, 0);
+                n = 0;
+            }
+            if (enter && cur >= 0) leave(n + __popc(fm & ((1u << lane) - 1u)));
+            n += __popc(fm);
+        }
+        if (enter) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int k = 0; k < 2 * NG; ++k) acc[i][k] = 0ull;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) pv[k] = 0.f;
+            cur = t;
+            j0 = i0;
+            j1 = i1;
+            j2 = i2;
+        }
+
+        cp_async_wait<2>();  // row yy (this lane's part)
+        const float4 r = in ? sh.rast[st][lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        // pixels that add nothing take zero barycentrics
+        const float bu = live ? r.x : 0.f, bv = live ? r.y : 0.f, bw = live ? 1.0f - r.x - r.y : 0.f;
+        const f32x2 uu = pack2(r.x, r.x), vv = pack2(r.y, r.y);
+        const f32x2 bb[3] = {pack2(bu, bu), pack2(bv, bv), pack2(bw, bw)};
+        float gu = 0.f, gv = 0.f, sr = 0.f;
+        const long long row = image_offset + (long long)pix * C;
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            ulonglong2 x0v = make_ulonglong2(0ull, 0ull), x1v = x0v, x2v = x0v, tv = x0v;
+            if (t >= 0) {
+                x0v = load_pairs<VEC>(A + (long long)i0 * C + 4 * g, C - 4 * g);
+                x1v = load_pairs<VEC>(A + (long long)i1 * C + 4 * g, C - 4 * g);
+                x2v = load_pairs<VEC>(A + (long long)i2 * C + 4 * g, C - 4 * g);
+            }
+            if (in) tv = *reinterpret_cast<const ulonglong2*>(&sh.target[st][g][lane]);
+            f32x2 val[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const f32x2 a0 = k ? x0v.y : x0v.x, a1 = k ? x1v.y : x1v.x, a2 = k ? x2v.y : x2v.x;
+                const f32x2 d0 = fma2(a2, minus1, a0), d1 = fma2(a2, minus1, a1);
+                val[k] = fma2(d0, uu, fma2(d1, vv, a2));
+                const f32x2 d = fma2(k ? tv.y : tv.x, minus1, val[k]);
+                sr += fabsf(lo2(d));
+                sr += fabsf(hi2(d));
+                const float g0 = l1_sign_fast(lo2(d), a.l1_scale), g1 = l1_sign_fast(hi2(d), a.l1_scale);
+                gu = fmaf(g1, hi2(d0), fmaf(g0, lo2(d0), gu));
+                gv = fmaf(g1, hi2(d1), fmaf(g0, lo2(d1), gv));
+                const f32x2 gg = pack2(g0, g1);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) acc[i][2 * g + k] = fma2(gg, bb[i], acc[i][2 * g + k]);
+            }
+            const float v4[4] = {lo2(val[0]), hi2(val[0]), lo2(val[1]), hi2(val[1])};
+            if (cl.plain & bit) store4<VEC>(a.out + row + 4 * g, C - 4 * g, v4);
+            if ((cl.listed & bit) && !a.emit_color)  // for the listed pixels' kernel
+                store4<VEC>(a.color + row + 4 * g, C - 4 * g, v4);
+        }
+        if (cl.plain & bit) s += sr;
+        if (live) {
+            float4 g3[3];
+            uv_grad_fast(P[i0], P[i1], P[i2], X, fmaf((float)(2 * yy + 1), rh, -1.0f), gu, gv, g3);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                pv[3 * i] += g3[i].x;
+                pv[3 * i + 1] += g3[i].y;
+                pv[3 * i + 2] += g3[i].w;
+            }
+        }
+        t = t_n;
+        t_n = t_nn;
+        i0 = n0;
+        i1 = n1;
+        i2 = n2;
+        pix += W;
+        st = st + 1 == kFitStages ? 0 : st + 1;
+    }
+    // what the columns still hold
+    const unsigned fm = __ballot_sync(0xffffffffu, cur >= 0);
+    if (n + __popc(fm) > 32) {
+        fit_drain<NG, true, VEC>(a, it, sh, n, 0);
+        n = 0;
+    }
+    if (cur >= 0) leave(n + __popc(fm & ((1u << lane) - 1u)));
+    n += __popc(fm);
+    if (n) fit_drain<NG, true, VEC>(a, it, sh, n, 0);
+    return s;
+}
+
+// The same for any channel count and alignment: each pixel's values are the
+// row (no sums held over rows: the registers hold eight channels at a time),
+// the 32 rows of a row of pixels are added at once.
+template <bool VEC>
+__device__ __forceinline__ float fit_rows(const BatchArgs& a, const drp_batch_item& it, FitWalkShared& sh, int x0,
+                                          int y0, int y1, const FitClass& cl) {
+    const int lane = threadIdx.x & 31, x = x0 + lane;
+    const int W = it.width, C = it.channels;
+    const bool in = x < W;
+    const float4* R = reinterpret_cast<const float4*>(a.rast) + it.pixel_offset;
+    const uint32_t* Wd = a.aa_words + it.pixel_offset;
+    const int* tri = a.tri + 3 * (long long)it.tri_first;
+    const float* A = a.attr + it.attr_offset;
+    const long long image_offset = it.image_offset;
+    const float X = fmaf((float)(2 * x + 1), __frcp_rn((float)W), -1.0f), rh = __frcp_rn((float)it.height);
+    const float sc = a.l1_scale;
+    float s = 0.f;
+    int pix = y0 * W + x;
+#pragma unroll 1
+    for (int yy = y0; yy < y1; ++yy, pix += W) {
+        const unsigned bit = 1u << (yy - y0);
+        const long long row = image_offset + (long long)pix * C;
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        float tv[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        int t = -1, i0 = 0, i1 = 0, i2 = 0;
+        if (in) {
+            t = (int)(Wd[pix] & ~kPixSil) - 1;
+            r = R[pix];
+            load4<VEC>(a.target + row, C, tv[0]);
+            if (C > 4) load4<VEC>(a.target + row + 4, C - 4, tv[1]);
+            if (t >= 0) {
+                i0 = tri[3 * (long long)t];
+                i1 = tri[3 * (long long)t + 1];
+                i2 = tri[3 * (long long)t + 2];
+            }
+        }
+        const bool plain = cl.plain & bit, live = cl.live & bit;
+        const bool keep_color = (cl.listed & bit) && !a.emit_color;  // for the listed pixels' kernel
+        const unsigned live_mask = __ballot_sync(0xffffffffu, live);
+        const int n = __popc(live_mask);
+        float* rw = sh.rows[__popc(live_mask & ((1u << lane) - 1u))];
+        if (live) *reinterpret_cast<int4*>(rw + 36) = make_int4(i0, i1, i2, 0);
+        const float u = r.x, v = r.y, w = 1.0f - u - v;
+        float gu = 0.f, gv = 0.f;
+#pragma unroll 1
+        for (int c0 = 0; c0 < C; c0 += 8) {
+            const int ng = C - c0 > 4 ? 2 : 1;
+            const bool last = c0 + 8 >= C;
+#pragma unroll
+            for (int gi = 0; gi < 2; ++gi) {
+                if (gi >= ng) break;
+                const int cg = c0 + 4 * gi;
+                float q0[4], q1[4], q2[4], val[4], g[4];
+                lerp_group<VEC>(A, C, cg, t, i0, i1, i2, u, v, q0, q1, q2, val);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float d = plain && (VEC || cg + k < C) ? val[k] - tv[gi][k] : 0.f;
+                    s += fabsf(d);
+                    g[k] = l1_sign_fast(d, sc);
+                }
+                if (plain) store4<VEC>(a.out + row + cg, C - cg, val);
+                if (keep_color) store4<VEC>(a.color + row + cg, C - cg, val);
+                if (in && cg + 8 < C) load4<VEC>(a.target + row + cg + 8, C - cg - 8, tv[gi]);
+                if (live) {
+                    float4* d = reinterpret_cast<float4*>(rw + 12 * gi);
+                    d[0] = make_float4(g[0] * u, g[1] * u, g[2] * u, g[3] * u);
+                    d[1] = make_float4(g[0] * v, g[1] * v, g[2] * v, g[3] * v);
+                    d[2] = make_float4(g[0] * w, g[1] * w, g[2] * w, g[3] * w);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        gu = fmaf(g[k], q0[k] - q2[k], gu);
+                        gv = fmaf(g[k], q1[k] - q2[k], gv);
+                    }
+                }
+            }
+            if (last && live) {
+                const float4* P = reinterpret_cast<const float4*>(a.pos) + it.pos_offset;
+                float4 g3[3];
+                uv_grad_fast(P[i0], P[i1], P[i2], X, fmaf((float)(2 * yy + 1), rh, -1.0f), gu, gv, g3);
+                float4* d = reinterpret_cast<float4*>(rw + 12 * ng);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) d[i] = make_float4(g3[i].x, g3[i].y, 0.f, g3[i].w);
+            }
+            if (!n) continue;
+            if (last && ng == 2) fit_drain<2, true, VEC>(a, it, sh, n, c0);
+            else if (last) fit_drain<1, true, VEC>(a, it, sh, n, c0);
+            else fit_drain<2, false, VEC>(a, it, sh, n, c0);
+        }
+    }
+    return s;
+}
+
+// One region of 32 x 16 pixels per CTA: WARPS warps of 16 / WARPS rows.
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) batch_fit_kernel(const __grid_constant__ BatchArgs a) {
+    constexpr int ROWS = 16 / WARPS;
+    __shared__ __align__(16) FitShared sh[WARPS];
+    __shared__ float warp_sum[WARPS];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int per_tile = fit_regions_per_tile(a.tile_log2);
+    const long long tile_id = blockIdx.x / per_tile;
+    const drp_batch_item& it = a.items[find_item_by_tile(a.items, a.num_items, tile_id)];
+    const int tile = (int)(tile_id - it.tile_offset);
+    const int ty = tile / it.tiles_x, tx = tile - ty * it.tiles_x;
+    const bool owner = a.tile_log2 == 5 || (a.tile_log2 == 4 ? (tx & 1) == 0 : (tx & 3) == 0 && (ty & 1) == 0);
+    const int warp = threadIdx.x >> 5;
+    const int x0 = tx << a.tile_log2;
+    const int y0 = (ty << a.tile_log2) + (int)(blockIdx.x % per_tile) * 16 + ROWS * warp;
+    const int y1 = min(y0 + ROWS, it.height);
+    float s = 0.f;
+    if (owner && y0 < y1) {
+        const bool vec = (it.channels & 3) == 0 &&
+                         ((reinterpret_cast<uintptr_t>(a.attr + it.attr_offset) |
+                           reinterpret_cast<uintptr_t>(a.grad_attr + it.attr_offset) |
+                           reinterpret_cast<uintptr_t>(a.target + it.image_offset) |
+                           reinterpret_cast<uintptr_t>(a.out + it.image_offset) |
+                           reinterpret_cast<uintptr_t>(a.color + it.image_offset)) & 15) == 0;
+        FitClass cl;
+        if (vec) s = fit_pairs<true, ROWS>(a, it, sh[warp].p, x0, y0, y1, cl);
+        else s = fit_pairs<false, ROWS>(a, it, sh[warp].p, x0, y0, y1, cl);
+        __syncwarp();  // the pair terms' shared memory becomes the walk's
+        // walks hold the sums of four or eight channels; see fit_rows
+        if (vec && it.channels == 8) s += fit_walk<2, true>(a, it, sh[warp].w, x0, y0, y1, cl);
+        else if (vec && it.channels == 4) s += fit_walk<1, true>(a, it, sh[warp].w, x0, y0, y1, cl);
+        else if (it.channels <= 4) s += fit_walk<1, false>(a, it, sh[warp].w, x0, y0, y1, cl);
+        else if (it.channels <= 8) s += fit_walk<2, false>(a, it, sh[warp].w, x0, y0, y1, cl);
+        else if (vec) s += fit_rows<true>(a, it, sh[warp].w, x0, y0, y1, cl);
+        else s += fit_rows<false>(a, it, sh[warp].w, x0, y0, y1, cl);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if ((threadIdx.x & 31) == 0) warp_sum[warp] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float sum = warp_sum[0];
+#pragma unroll
+        for (int k = 1; k < WARPS; ++k) sum += warp_sum[k];
+        *fit_loss_slot(a, blockIdx.x) = sum;
+        if (it.channels > 32) atomicOr(a.stats + 2, DRP_DEVERR_CHANNELS);
+    }
+}
+
 // The backward of one pixel no blending pair touches, with the upstream
 // gradient sign(out - target) * scale given by the sign masks (bit c:
 // nonzero / positive): interpolation backward (attribute gradients) and
@@ -788,10 +1558,11 @@ __device__ __forceinline__ void pixel_backward_l1(const BatchArgs& a, const drp_
     }
 }
 
-// Antialias + L1 loss with the loss's gradient formed in the same pass
-// (drp_batch_forward_l1_grad).  Every pixel: its output and |error| partial
+// Antialias + L1 loss with the loss's gradient formed in the same pass, one
+// thread per pixel, from a stored colour image: the form for launches below
+// kFitPixels (batch_fit_kernel above).  Every pixel: its output and |error| partial
 // as batch_aa_l1_kernel computes them.  Then, for the pixels no blending pair
-// touches (the listed ones belong to batch_aa_bwd_kernel<true>, which forms
+// touches (the listed ones belong to batch_aa_bwd_kernel, which forms
 // the sign from the output and the target), the pixel's whole backward with
 // the upstream gradient sign(out - target) * scale: interpolation backward
 // (attribute gradients) and rasterisation backward (vertex gradients),
@@ -849,6 +1620,34 @@ __global__ void __launch_bounds__(256, 4) batch_aa_l1_grad_kernel(BatchArgs a) {
     }
 }
 
+// Interpolated colours of every pixel from its rast row: what the fine raster
+// stores when it is asked to, for a backward that needs them after
+// drp_batch_fit_l1 kept none.  Bound by its rast reads and colour writes.
+__global__ void __launch_bounds__(256) batch_color_kernel(BatchArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int2 blk = a.pix_blocks[blockIdx.x];
+    const drp_batch_item& it = a.items[blk.x];
+    const int pix = blk.y * 256 + threadIdx.x, C = it.channels;
+    if (pix >= it.width * it.height) return;
+    const float4 r = reinterpret_cast<const float4*>(a.rast)[it.pixel_offset + pix];
+    int i0 = 0, i1 = 0, i2 = 0;
+    const int t = checked_tri(r.w, a.tri + 3 * (long long)it.tri_first, it.tri_count, it.num_vertices, i0, i1, i2);
+    const float* A = a.attr + it.attr_offset;
+    float* o = a.color + it.image_offset + (long long)pix * C;
+    const bool vec = (C & 3) == 0 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(o)) & 15) == 0;
+    for (int c = 0; c < C; c += 4) {
+        float x0[4], x1[4], x2[4], v[4];
+        if (vec) {
+            lerp_group<true>(A, C, c, t, i0, i1, i2, r.x, r.y, x0, x1, x2, v);
+            store4<true>(o + c, C - c, v);
+        } else {
+            lerp_group<false>(A, C, c, t, i0, i1, i2, r.x, r.y, x0, x1, x2, v);
+            store4<false>(o + c, C - c, v);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Host side.
 // ---------------------------------------------------------------------------
@@ -875,19 +1674,22 @@ BatchLayout batch_layout(long long total_prims, long long total_tiles, unsigned 
 }
 
 // Antialias state block: list count at 0, per-pixel flags at 256, the pixel
-// list (int32) after them.
-static size_t aa_state_bytes(long long total_pixels, size_t* list_off) {
-    const size_t flags_end = 256 + (size_t)total_pixels;
-    const size_t lo = (flags_end + 255) / 256 * 256;
+// list (int32) after them, then the pixel words.
+static size_t aa_state_bytes(long long total_pixels, size_t* list_off, size_t* words_off) {
+    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    const size_t lo = up(256 + (size_t)total_pixels);
+    const size_t wo = up(lo + (size_t)total_pixels * 4);
     if (list_off) *list_off = lo;
-    return lo + (size_t)total_pixels * 4;
+    if (words_off) *words_off = wo;
+    return wo + (size_t)total_pixels * 4;
 }
 
 static void carve_aa_state(BatchArgs& a, void* state, long long total_pixels) {
     if (!state) return;
-    size_t lo = 0;
-    aa_state_bytes(total_pixels, &lo);
+    size_t lo = 0, wo = 0;
+    aa_state_bytes(total_pixels, &lo, &wo);
     char* p = static_cast<char*>(state);
+    a.aa_words = reinterpret_cast<uint32_t*>(p + wo);
     a.aa_count = reinterpret_cast<unsigned*>(p);
     a.aa_flags = reinterpret_cast<unsigned char*>(p + 256);
     a.aa_list = reinterpret_cast<int*>(p + lo);
@@ -897,6 +1699,7 @@ static void carve(BatchArgs& a, void* ws, const BatchLayout& L) {
     char* w = static_cast<char*>(ws);
     a.stats = reinterpret_cast<uint32_t*>(w + L.stats);
     a.queue = reinterpret_cast<uint32_t*>(w + L.queue);
+    a.loss_count = a.stats + 32;  // in the stats block, zeroed with it
     a.prims = reinterpret_cast<int4*>(w + L.prims);
     a.tile_count = reinterpret_cast<uint32_t*>(w + L.count);
     a.tile_offset = reinterpret_cast<uint32_t*>(w + L.offset);
@@ -905,6 +1708,12 @@ static void carve(BatchArgs& a, void* ws, const BatchLayout& L) {
     a.chunk_sums = reinterpret_cast<unsigned long long*>(w + L.chunks);
     a.aa_rec = reinterpret_cast<float4*>(w + L.aa);
 }
+
+// Rows per warp: a walk of eight adds fewest sums per pixel, but below this
+// many regions two warps each leave the chip idle, and four rows per warp are
+// faster (one 1024 x 1024 view, 2048 regions: 126.7 against 129.5 us per step;
+// 64 views of 512 x 512, 32768 regions: 1039 against 946 us).
+constexpr long long kFitTallRegions = 4096;
 
 // Up to this many tiles per resident fine CTA the work order is sorted.
 constexpr long long kOrderTilesPerCTA = 8;
@@ -938,7 +1747,7 @@ __global__ void __launch_bounds__(256) batch_clear_kernel(uint32_t* stats, unsig
     }
 }
 
-template <int TL, int TPT>
+template <int TL, int TPT, bool FIT>
 static void launch_batch_fine(const BatchArgs& a, cudaStream_t s) {
     constexpr int NT = (1 << (2 * TL)) < 256 ? (1 << (2 * TL)) : 256;
     // persistent grid: every resident CTA slot of the device (occupancy per
@@ -946,7 +1755,7 @@ static void launch_batch_fine(const BatchArgs& a, cudaStream_t s) {
     static std::atomic<int> per_sm{0};
     int per = per_sm.load(std::memory_order_relaxed);
     if (per == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_fine_kernel<TL, TPT>, NT, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_fine_kernel<TL, TPT, FIT>, NT, 0);
         per = per > 0 ? per : 1;
         per_sm.store(per, std::memory_order_relaxed);
     }
@@ -962,8 +1771,21 @@ static void launch_batch_fine(const BatchArgs& a, cudaStream_t s) {
         launch_tile_order(a.tile_count, a.total_tiles, a.tile_cursor, s);
         b.tile_order = a.tile_cursor;
     }
-    launch_pdl(batch_fine_kernel<TL, TPT>, dim3((unsigned)g), dim3(NT), s, b);
+    launch_pdl(batch_fine_kernel<TL, TPT, FIT>, dim3((unsigned)g), dim3(NT), s, b);
     drp_note_launch();
+}
+
+template <int TL, bool FIT>
+static void launch_batch_fine(const BatchArgs& a, cudaStream_t s) {
+    switch (a.tpt) {
+    case 0: launch_batch_fine<TL, 0, FIT>(a, s); break;
+    case 1: launch_batch_fine<TL, 1, FIT>(a, s); break;
+    case 2: launch_batch_fine<TL, 2, FIT>(a, s); break;
+    case 4: launch_batch_fine<TL, 4, FIT>(a, s); break;
+    case 8: launch_batch_fine<TL, 8, FIT>(a, s); break;
+    case 16: launch_batch_fine<TL, 16, FIT>(a, s); break;
+    default: launch_batch_fine<TL, 32, FIT>(a, s); break;
+    }
 }
 
 template <int TL>
@@ -983,15 +1805,8 @@ static void launch_batch_raster(const BatchArgs& a, cudaStream_t s) {
     } else {
         cudaMemsetAsync(a.tile_offset, 0, sizeof(uint32_t) * a.total_tiles, s);
     }
-    switch (a.tpt) {
-    case 0: launch_batch_fine<TL, 0>(a, s); break;
-    case 1: launch_batch_fine<TL, 1>(a, s); break;
-    case 2: launch_batch_fine<TL, 2>(a, s); break;
-    case 4: launch_batch_fine<TL, 4>(a, s); break;
-    case 8: launch_batch_fine<TL, 8>(a, s); break;
-    case 16: launch_batch_fine<TL, 16>(a, s); break;
-    default: launch_batch_fine<TL, 32>(a, s); break;
-    }
+    if (a.fit) launch_batch_fine<TL, true>(a, s);
+    else launch_batch_fine<TL, false>(a, s);
 }
 
 // A side stream with its fork / join events, one per host thread and device,
@@ -1058,12 +1873,24 @@ int launch_batch_forward(BatchArgs a, void* ws, const BatchLayout& L, cudaStream
     // (the antialias triangle records were written by the setup / count pass)
     if (a.target && a.l1_grads) {
         if (a.n_pix_blocks > 0) {
-            launch_pdl(batch_aa_l1_grad_kernel, dim3((unsigned)a.n_pix_blocks), dim3(256), s, a);
+            if (a.fit) {
+                const long long regions = a.total_tiles * fit_regions_per_tile(a.tile_log2);
+                if (regions < kFitTallRegions)
+                    launch_pdl(batch_fit_kernel<4>, dim3((unsigned)regions), dim3(128), s, a);
+                else
+                    launch_pdl(batch_fit_kernel<2>, dim3((unsigned)regions), dim3(64), s, a);
+            } else {
+                launch_pdl(batch_aa_l1_grad_kernel, dim3((unsigned)a.n_pix_blocks), dim3(256), s, a);
+            }
             drp_note_launch();
             // the listed pixels' whole backward, and (its last block) the
             // final loss sum: one launch on the chain
-            const long long g = list_kernel_grid<true>(a.n_pix_blocks);
-            launch_pdl(batch_aa_bwd_kernel<true, kListLanes>, dim3((unsigned)g), dim3(256), s, a);
+            if (a.fit)
+                launch_pdl(batch_aa_bwd_kernel<kListFit, kListLanes>,
+                           dim3((unsigned)list_kernel_grid<kListFit>(a.n_pix_blocks)), dim3(256), s, a);
+            else
+                launch_pdl(batch_aa_bwd_kernel<kListL1, kListLanes>,
+                           dim3((unsigned)list_kernel_grid<kListL1>(a.n_pix_blocks)), dim3(256), s, a);
             drp_note_launch();
         } else {
             launch_l1_final(a.block_loss, a.n_pix_blocks, a.l1_scale, a.loss, s);
@@ -1102,7 +1929,7 @@ int launch_batch_backward(BatchArgs a, void* ws, const BatchLayout& L, bool reus
     // and the fused backward of all other pixels are independent: fork the
     // list kernel onto a side stream so it fills the SMs beside the main
     // kernel and its tail, then join.  Both only add into the gradients.
-    const long long g = list_kernel_grid<false>(a.n_pix_blocks);
+    const long long g = list_kernel_grid<kListBackward>(a.n_pix_blocks);
     SideStream side;
     const bool fork = side_stream(s, side);
     if (fork) {
@@ -1111,7 +1938,7 @@ int launch_batch_backward(BatchArgs a, void* ws, const BatchLayout& L, bool reus
     }
     batch_bwd_kernel<<<(unsigned)a.n_pix_blocks, 256, 0, s>>>(a);
     drp_note_launch();
-    batch_aa_bwd_kernel<false, kListLanes><<<(unsigned)g, 256, 0, fork ? side.stream : s>>>(a);
+    batch_aa_bwd_kernel<kListBackward, kListLanes><<<(unsigned)g, 256, 0, fork ? side.stream : s>>>(a);
     drp_note_launch();
     if (fork) {
         cudaEventRecord(side.join, side.stream);
@@ -1187,7 +2014,7 @@ DRP_API int drp_batch_block_maps(const drp_batch_item* items, int num_items, int
 
 DRP_API int drp_batch_aa_state_size(long long total_pixels, size_t* bytes) {
     if (!bytes || total_pixels <= 0) return bfail("drp_batch_aa_state_size: bad arguments");
-    *bytes = drp::aa_state_bytes(total_pixels, nullptr);
+    *bytes = drp::aa_state_bytes(total_pixels, nullptr, nullptr);
     return DRP_STATUS_OK;
 }
 
@@ -1307,15 +2134,15 @@ DRP_API int drp_batch_forward_l1(void* workspace, size_t workspace_bytes, const 
     return drp_check_launch("drp_batch_forward_l1");
 }
 
-DRP_API int drp_batch_forward_l1_grad(void* workspace, size_t workspace_bytes, const drp_batch_item* items,
-                                      int num_items, const int* prim_block_map, long long prim_blocks,
-                                      const int* pixel_block_map, long long pixel_blocks, long long total_prims,
-                                      long long total_tiles, const float* pos, const int* tri, const float* attr,
-                                      const int* nbr, int tile_log2, int threads_per_tri,
-                                      unsigned long long list_capacity, unsigned bin_depth, float* rast, float* color,
-                                      float* out, void* aa_state, long long total_pixels, const float* target,
-                                      float scale, float* block_loss, float* loss, float* grad_pos, float* grad_attr,
-                                      float* zero_first, long long zero_floats, void* stream) {
+static int batch_fit_l1(const char* who, bool full_color, void* workspace, size_t workspace_bytes, const drp_batch_item* items,
+                        int num_items, const int* prim_block_map, long long prim_blocks,
+                        const int* pixel_block_map, long long pixel_blocks, long long total_prims,
+                        long long total_tiles, const float* pos, const int* tri, const float* attr,
+                        const int* nbr, int tile_log2, int threads_per_tri,
+                        unsigned long long list_capacity, unsigned bin_depth, float* rast, float* color,
+                        float* out, void* aa_state, long long total_pixels, const float* target,
+                        float scale, float* block_loss, float* loss, float* grad_pos, float* grad_attr,
+                        float* zero_first, long long zero_floats, void* stream) {
     drp::BatchArgs a;
     drp::BatchLayout L;
     int st = batch_common(workspace, workspace_bytes, items, num_items, prim_block_map, prim_blocks, pixel_block_map,
@@ -1341,6 +2168,8 @@ DRP_API int drp_batch_forward_l1_grad(void* workspace, size_t workspace_bytes, c
     a.color = color;
     a.out = out;
     carve_aa_state(a, aa_state, total_pixels);
+    a.fit = total_pixels >= drp::kFitPixels;
+    a.emit_color = full_color;  // else the loss pass stores the listed pixels' colours only
     a.emit_out = false;  // the fused antialias + loss pass writes every output pixel
     a.aa_records = true;
     a.target = target;
@@ -1356,7 +2185,58 @@ DRP_API int drp_batch_forward_l1_grad(void* workspace, size_t workspace_bytes, c
     a.zero_first = zero_floats > 0 ? zero_first : nullptr;
     a.zero_floats = zero_floats;
     drp::launch_batch_forward(a, workspace, L, static_cast<cudaStream_t>(stream));
-    return drp_check_launch("drp_batch_forward_l1_grad");
+    return drp_check_launch(who);
+}
+
+DRP_API int drp_batch_forward_l1_grad(void* workspace, size_t workspace_bytes, const drp_batch_item* items,
+                                      int num_items, const int* prim_block_map, long long prim_blocks,
+                                      const int* pixel_block_map, long long pixel_blocks, long long total_prims,
+                                      long long total_tiles, const float* pos, const int* tri, const float* attr,
+                                      const int* nbr, int tile_log2, int threads_per_tri,
+                                      unsigned long long list_capacity, unsigned bin_depth, float* rast, float* color,
+                                      float* out, void* aa_state, long long total_pixels, const float* target,
+                                      float scale, float* block_loss, float* loss, float* grad_pos, float* grad_attr,
+                                      float* zero_first, long long zero_floats, void* stream) {
+    return batch_fit_l1("drp_batch_forward_l1_grad", true, workspace, workspace_bytes, items, num_items, prim_block_map, prim_blocks, pixel_block_map, pixel_blocks,
+                       total_prims, total_tiles, pos, tri, attr, nbr, tile_log2, threads_per_tri, list_capacity, bin_depth,
+                       rast, color, out, aa_state, total_pixels, target, scale, block_loss, loss, grad_pos, grad_attr,
+                       zero_first, zero_floats, stream);
+}
+
+DRP_API int drp_batch_fit_l1(void* workspace, size_t workspace_bytes, const drp_batch_item* items,
+                             int num_items, const int* prim_block_map, long long prim_blocks,
+                             const int* pixel_block_map, long long pixel_blocks, long long total_prims,
+                             long long total_tiles, const float* pos, const int* tri, const float* attr,
+                             const int* nbr, int tile_log2, int threads_per_tri,
+                             unsigned long long list_capacity, unsigned bin_depth, float* rast, float* color,
+                             float* out, void* aa_state, long long total_pixels, const float* target,
+                             float scale, float* block_loss, float* loss, float* grad_pos, float* grad_attr,
+                             float* zero_first, long long zero_floats, void* stream) {
+    return batch_fit_l1("drp_batch_fit_l1", false, workspace, workspace_bytes, items, num_items, prim_block_map, prim_blocks, pixel_block_map, pixel_blocks,
+                       total_prims, total_tiles, pos, tri, attr, nbr, tile_log2, threads_per_tri, list_capacity, bin_depth,
+                       rast, color, out, aa_state, total_pixels, target, scale, block_loss, loss, grad_pos, grad_attr,
+                       zero_first, zero_floats, stream);
+}
+
+DRP_API int drp_batch_colors(const drp_batch_item* items, int num_items, const int* pixel_block_map,
+                             long long pixel_blocks, const int* tri, const float* attr, const float* rast,
+                             float* color, void* stream) {
+    if (!items || num_items <= 0 || !tri || !attr || !rast || !color || (reinterpret_cast<uintptr_t>(rast) & 15) ||
+        pixel_blocks < 0 || pixel_blocks > 0x7fffffffll || (pixel_blocks > 0 && !pixel_block_map))
+        return bfail("drp_batch_colors: bad table or buffers");
+    if (pixel_blocks == 0) return DRP_STATUS_OK;
+    drp::BatchArgs a{};
+    a.items = items;
+    a.num_items = num_items;
+    a.pix_blocks = reinterpret_cast<const int2*>(pixel_block_map);
+    a.tri = tri;
+    a.attr = attr;
+    a.rast = const_cast<float*>(rast);
+    a.color = color;
+    drp::launch_pdl(drp::batch_color_kernel, dim3((unsigned)pixel_blocks), dim3(256),
+                    static_cast<cudaStream_t>(stream), a);
+    drp_note_launch();
+    return drp_check_launch("drp_batch_colors");
 }
 
 DRP_API int drp_batch_backward(void* workspace, size_t workspace_bytes, const drp_batch_item* items, int num_items,

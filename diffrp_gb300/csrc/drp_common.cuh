@@ -412,6 +412,48 @@ __device__ __forceinline__ void atomic_add4(float4* dst, const float4& v) {
 #endif
 }
 
+// Asynchronous copy of N bytes (4 or 16, both ends aligned to N) into shared
+// memory; a thread's copies since its last commit form a group, and wait<K>
+// returns when all but its last K groups have arrived (visible to that thread).
+template <int N>
+__device__ __forceinline__ void cp_async(void* dst, const void* src) {
+    static_assert(N == 4 || N == 16, "cp_async: 4 or 16 bytes");
+#if defined(__CUDA_ARCH__)
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(N) : "memory");
+#else
+    memcpy(dst, src, N);
+#endif
+}
+__device__ __forceinline__ void cp_async_commit() {
+#if defined(__CUDA_ARCH__)
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#endif
+}
+template <int K>
+__device__ __forceinline__ void cp_async_wait() {
+#if defined(__CUDA_ARCH__)
+    asm volatile("cp.async.wait_group %0;" ::"n"(K) : "memory");
+#endif
+}
+
+// Two floats per instruction (sm_100 and later): each half rounds as fmaf.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    return ((f32x2)__float_as_uint(hi) << 32) | (f32x2)__float_as_uint(lo);
+}
+__device__ __forceinline__ float lo2(f32x2 a) { return __uint_as_float((uint32_t)a); }
+__device__ __forceinline__ float hi2(f32x2 a) { return __uint_as_float((uint32_t)(a >> 32)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+#if defined(__CUDA_ARCH__)
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+#else
+    return pack2(fmaf(lo2(a), lo2(b), lo2(c)), fmaf(hi2(a), hi2(b), hi2(c)));
+#endif
+}
+
 // s + x exactly as a float pair: s' = fl(s + x), err = (s + x) - s' (Knuth's
 // TwoSum, no branch).  Sums of pairs carry their rounding errors in c.
 __device__ __forceinline__ void two_sum(float& s, float& c, float x) {
@@ -425,26 +467,14 @@ __device__ __forceinline__ void two_sum(float& s, float& c, float x) {
 // Threads of the block that forms a loss from its per-block partials.
 constexpr int kFinalThreads = 256;
 
-// *loss = scale * (sum of nblocks partials), by one whole block of NT
-// threads: every thread adds its strided elements (eight loads in flight)
-// in index order as a (sum, error) float pair, then the pairs are combined
-// by a fixed shuffle tree within warps and across them -- a fixed order, so
-// the loss is reproducible from run to run.  Float pairs instead of doubles:
-// FP64 issues at a small fraction of the FP32 rate on this part, and this
-// block sits on the step's critical path.  Every thread of the block calls
-// it (it has a barrier).
+// *out = scale * (sum of the block's (s, c) float pairs), by one whole block of
+// NT threads: a fixed shuffle tree within warps and across them.  Every thread
+// of the block calls it (it has a barrier, and one before it may be called
+// again is the caller's).
 template <int NT>
-__device__ __forceinline__ void l1_final_block(const float* partial, long long nblocks, float scale, float* loss) {
-    static_assert(NT % 32 == 0 && NT <= 1024, "l1_final_block: whole warps, at most 1024 threads");
+__device__ __forceinline__ void block_sum_pairs(float s, float c, float scale, float* out) {
+    static_assert(NT % 32 == 0 && NT <= 1024, "block_sum_pairs: whole warps, at most 1024 threads");
     __shared__ float warp_s[NT / 32], warp_c[NT / 32];
-    float s = 0.0f, c = 0.0f;
-    for (long long i = threadIdx.x; i < nblocks; i += 8 * NT) {
-        float v[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = i + k * NT < nblocks ? partial[i + k * NT] : 0.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) two_sum(s, c, v[k]);
-    }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         const float os = __shfl_xor_sync(0xffffffffu, s, off), oc = __shfl_xor_sync(0xffffffffu, c, off);
@@ -465,8 +495,29 @@ __device__ __forceinline__ void l1_final_block(const float* partial, long long n
             w += ow;
             two_sum(v, w, ov);
         }
-        if (threadIdx.x == 0) *loss = (v + w) * scale;
+        if (threadIdx.x == 0) *out = (v + w) * scale;
     }
+}
+
+// *loss = scale * (sum of nblocks partials), by one whole block of NT
+// threads: every thread adds its strided elements (eight loads in flight)
+// in index order as a (sum, error) float pair, then the pairs are combined
+// by a fixed shuffle tree within warps and across them -- a fixed order, so
+// the loss is reproducible from run to run.  Float pairs instead of doubles:
+// FP64 issues at a small fraction of the FP32 rate on this part, and this
+// block sits on the step's critical path.  Every thread of the block calls
+// it (it has a barrier).
+template <int NT>
+__device__ __forceinline__ void l1_final_block(const float* partial, long long nblocks, float scale, float* loss) {
+    float s = 0.0f, c = 0.0f;
+    for (long long i = threadIdx.x; i < nblocks; i += 8 * NT) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = i + k * NT < nblocks ? partial[i + k * NT] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) two_sum(s, c, v[k]);
+    }
+    block_sum_pairs<NT>(s, c, scale, loss);
 }
 
 }  // namespace drp

@@ -404,7 +404,7 @@ int drp_batch_workspace_size(long long total_prims, long long total_tiles, unsig
  * raises the u32 at byte 12 to its count.
  * aa_state (may be NULL; drp_batch_aa_state_size(total_pixels) bytes,
  * 256-byte aligned): the antialias pass records there which pixels a
- * blending pair touches (a flag per pixel and a list of them), so that
+ * blending pair touches (a flag per pixel and a list of them, with scratch), so that
  * drp_batch_backward evaluates the antialias terms of those pixels only.
  */
 int drp_batch_forward(void* workspace, size_t workspace_bytes, const drp_batch_item* items, int num_items,
@@ -463,6 +463,31 @@ int drp_batch_forward_l1_grad(void* workspace, size_t workspace_bytes, const drp
                               float* out, void* aa_state, long long total_pixels, const float* target, float scale,
                               float* block_loss, float* loss, float* grad_pos, float* grad_attr, float* zero_first,
                               long long zero_floats, void* stream);
+
+/*
+ * drp_batch_forward_l1_grad without the colour image: color (image floats)
+ * is scratch, of which a large launch writes only the unblended colours of
+ * the pixels a blending pair touches (the other pixels' colours are
+ * interpolated where they are needed and never stored).  All other arguments, outputs and
+ * limits are drp_batch_forward_l1_grad's.  No counterpart in the reference.
+ */
+int drp_batch_fit_l1(void* workspace, size_t workspace_bytes, const drp_batch_item* items, int num_items,
+                     const int* prim_block_map, long long prim_blocks, const int* pixel_block_map,
+                     long long pixel_blocks, long long total_prims, long long total_tiles, const float* pos,
+                     const int* tri, const float* attr, const int* nbr, int tile_log2, int threads_per_tri,
+                     unsigned long long list_capacity, unsigned bin_depth, float* rast, float* color, float* out,
+                     void* aa_state, long long total_pixels, const float* target, float scale, float* block_loss,
+                     float* loss, float* grad_pos, float* grad_attr, float* zero_first, long long zero_floats,
+                     void* stream);
+
+/*
+ * The interpolated colours (image floats, item layout) of every pixel from its
+ * rast row, as drp_batch_forward writes them: for a caller of
+ * drp_batch_fit_l1 that needs them after all (drp_batch_backward's color).
+ * No counterpart in the reference.
+ */
+int drp_batch_colors(const drp_batch_item* items, int num_items, const int* pixel_block_map, long long pixel_blocks,
+                     const int* tri, const float* attr, const float* rast, float* color, void* stream);
 
 /*
  * dst[i] = src[i] * scale[0] for n floats (scale: one device float), dst and
