@@ -124,13 +124,14 @@ def call(name, *args):
 _sizes = {}
 
 
-def size_out(name, *args):
-    """A workspace-size query (a pure function of its integer arguments),
-    answered from a cache after the first call."""
+def size_out(name, *args, ctype=ctypes.c_size_t):
+    """A size query (a pure function of its integer arguments, written
+    through an out-pointer of ``ctype``), answered from a cache after the
+    first call."""
     key = (name,) + args
     v = _sizes.get(key)
     if v is None:
-        out = ctypes.c_size_t(0)
+        out = ctype(0)
         call(name, *args, ctypes.byref(out))
         v = _sizes[key] = out.value
     return v

@@ -145,6 +145,9 @@ DRP_FAST(drp_antialias_fwd)
 DRP_FAST(drp_antialias_bwd)
 DRP_FAST(drp_edge_gradient_bwd)
 DRP_FAST(drp_l1_loss_fwd)
+DRP_FAST(drp_texture_mip_build)
+DRP_FAST(drp_texture_fwd)
+DRP_FAST(drp_texture_bwd)
 DRP_FAST(drp_transform_points_fwd)
 DRP_FAST(drp_transform_points_bwd)
 DRP_FAST(drp_copy_async)
@@ -157,12 +160,31 @@ DRP_FAST(drp_scale_floats)
 DRP_FAST(drp_batch_backward)
 
 PyMethodDef methods[] = {
-    DRP_ENTRY(drp_rasterize_fwd),     DRP_ENTRY(drp_rasterize_bwd),       DRP_ENTRY(drp_interpolate_fwd),
-    DRP_ENTRY(drp_interpolate_bwd),   DRP_ENTRY(drp_interpolate_sparse_fwd), DRP_ENTRY(drp_interpolate_sparse_bwd),
-    DRP_ENTRY(drp_antialias_topology), DRP_ENTRY(drp_antialias_fwd),      DRP_ENTRY(drp_antialias_bwd),
-    DRP_ENTRY(drp_edge_gradient_bwd), DRP_ENTRY(drp_l1_loss_fwd),         DRP_ENTRY(drp_batch_forward),
-    DRP_ENTRY(drp_batch_forward_l1),  DRP_ENTRY(drp_batch_forward_l1_grad),  DRP_ENTRY(drp_batch_fit_l1),  DRP_ENTRY(drp_batch_colors),  DRP_ENTRY(drp_scale_floats),  DRP_ENTRY(drp_batch_backward),      DRP_ENTRY(drp_transform_points_fwd),
-    DRP_ENTRY(drp_transform_points_bwd), DRP_ENTRY(drp_copy_async), {nullptr, nullptr, 0, nullptr}};
+    DRP_ENTRY(drp_rasterize_fwd),
+    DRP_ENTRY(drp_rasterize_bwd),
+    DRP_ENTRY(drp_interpolate_fwd),
+    DRP_ENTRY(drp_interpolate_bwd),
+    DRP_ENTRY(drp_interpolate_sparse_fwd),
+    DRP_ENTRY(drp_interpolate_sparse_bwd),
+    DRP_ENTRY(drp_antialias_topology),
+    DRP_ENTRY(drp_antialias_fwd),
+    DRP_ENTRY(drp_antialias_bwd),
+    DRP_ENTRY(drp_edge_gradient_bwd),
+    DRP_ENTRY(drp_l1_loss_fwd),
+    DRP_ENTRY(drp_texture_mip_build),
+    DRP_ENTRY(drp_texture_fwd),
+    DRP_ENTRY(drp_texture_bwd),
+    DRP_ENTRY(drp_transform_points_fwd),
+    DRP_ENTRY(drp_transform_points_bwd),
+    DRP_ENTRY(drp_copy_async),
+    DRP_ENTRY(drp_batch_forward),
+    DRP_ENTRY(drp_batch_forward_l1),
+    DRP_ENTRY(drp_batch_forward_l1_grad),
+    DRP_ENTRY(drp_batch_fit_l1),
+    DRP_ENTRY(drp_batch_colors),
+    DRP_ENTRY(drp_scale_floats),
+    DRP_ENTRY(drp_batch_backward),
+    {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_drp_fast", "CPython fast path onto libdiffrp_gb300", -1, methods,
                       nullptr, nullptr, nullptr, nullptr};

@@ -594,15 +594,12 @@ _TEX_BOUNDARIES = {"wrap": 0, "clamp": 1, "zero": 2, "mirror": 3}
 
 
 def _tex_levels(H, W, max_mip_level):
-    n = ctypes.c_int(0)
-    _ffi.call("drp_texture_levels", H, W, -1 if max_mip_level is None else int(max_mip_level), ctypes.byref(n))
-    return n.value
+    return _ffi.size_out("drp_texture_levels", H, W, -1 if max_mip_level is None else int(max_mip_level),
+                         ctype=ctypes.c_int)
 
 
 def _tex_pyramid_floats(N, H, W, C, levels):
-    n = ctypes.c_longlong(0)
-    _ffi.call("drp_texture_pyramid_floats", N, H, W, C, levels, ctypes.byref(n))
-    return n.value
+    return _ffi.size_out("drp_texture_pyramid_floats", N, H, W, C, levels, ctype=ctypes.c_longlong)
 
 
 def _tex_build(tex, levels):
