@@ -56,6 +56,8 @@ def _register():
         "drp_batch_aa_state_size": [LL, ctypes.POINTER(ctypes.c_size_t)],
         "drp_batch_forward": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL, ctypes.c_uint,
                               P, P, P, P, LL, P],
+        "drp_batch_render": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL, ctypes.c_uint,
+                             P, P, P, LL, P],
         "drp_batch_forward_l1": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL,
                                  ctypes.c_uint, P, P, P, P, LL, P, ctypes.c_float, P, P, P, P],
         "drp_batch_forward_l1_grad": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL,
@@ -306,7 +308,8 @@ class BatchRenderer:
         last, when it is not None; color is scratch then, written only at
         the pixels a blending pair touches).  flags: an
         antialias state block (_flags()) the forward fills for its backward,
-        or None."""
+        or None.  color=None (drp_batch_render): the images alone, for no
+        backward; flags is one word per pixel of scratch then."""
         if not torch.cuda.is_current_stream_capturing():
             self._poll_stats()
         first = not self._capacity
@@ -318,6 +321,7 @@ class BatchRenderer:
         optr = None if out is None else out.data_ptr()
         fptr = None if flags is None else flags.data_ptr()
         npix = self.total_pixels
+        bufs = (rast.data_ptr(), None if color is None else color.data_ptr(), optr, fptr, npix)
         self._fwd_gen += 1
         ws = self._workspace(cap)
         stream = _ffi.stream_of(self.device)
@@ -338,11 +342,14 @@ class BatchRenderer:
             tail = (target.data_ptr(), ctypes.c_float(scale), grad.data_ptr(), block_loss.data_ptr(),
                     loss.data_ptr(), stream)
             entry = "drp_batch_forward_l1"
+        elif color is None:
+            bufs = (rast.data_ptr(), fptr, optr, npix)
+            tail = (stream,)
+            entry = "drp_batch_render"
         else:
             tail = (stream,)
             entry = "drp_batch_forward"
-        _ffi.call(entry, ws.data_ptr(), ws.numel(), *args, cap, depth, rast.data_ptr(), color.data_ptr(), optr,
-                  fptr, npix, *tail)
+        _ffi.call(entry, ws.data_ptr(), ws.numel(), *args, cap, depth, *bufs, *tail)
         if first:
             # exact lists, sized synchronously; they also give the largest tile
             torch.cuda.current_stream(self.device).synchronize()
@@ -356,8 +363,7 @@ class BatchRenderer:
             self._depth = self._choose_depth(self.last_max_tile, needed)
             if needed > cap:
                 ws = self._workspace(self._capacity)
-                _ffi.call(entry, ws.data_ptr(), ws.numel(), *args, self._capacity, 0, rast.data_ptr(),
-                          color.data_ptr(), optr, fptr, npix, *tail)
+                _ffi.call(entry, ws.data_ptr(), ws.numel(), *args, self._capacity, 0, *bufs, *tail)
         else:
             self._queue_stats(ws)
         if out is not None or l1 is not None:  # a raster-only forward writes no AA records
@@ -397,7 +403,8 @@ class BatchRenderer:
             raise RuntimeError("pos must be a float32 CUDA tensor of shape (%d, 4)" % self.pos_rows)
         if attr.numel() != self.attr_floats or attr.dtype != torch.float32 or not attr.is_cuda:
             raise RuntimeError("attr must hold %d float32 values on the GPU" % self.attr_floats)
-        return _BatchFn.apply(pos.contiguous(), attr.contiguous().reshape(-1), self)
+        keep = torch.is_grad_enabled() and (pos.requires_grad or attr.requires_grad)
+        return _BatchFn.apply(pos.contiguous(), attr.contiguous().reshape(-1), self, keep)
 
     def render_l1(self, pos, attr, target, grads_in_forward=False):
         """Render and score in one pass: returns (loss, images) with loss =
@@ -451,15 +458,23 @@ def _chunk_views(r, fl, chunk, l1):
 
 class _BatchFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, pos, attr, renderer):
+    def forward(ctx, pos, attr, renderer, keep):
+        """keep: a backward may follow, so rast, colours and antialias state
+        are kept (or, with recompute, made again then)."""
         ctx.renderer = renderer
-        if renderer.recompute:
+        if renderer.recompute or not keep:
             out = torch.empty(renderer.image_floats, dtype=torch.float32, device=pos.device)
-            rast, fl, flags, _ = renderer._chunk_scratch(l1=False)
-            for c in renderer._chunks:
-                color, _ = _chunk_views(renderer, fl, c, False)
-                c.renderer._forward_raw(pos[c.rows], attr, rast, color, out[c.floats], flags=flags)
-            ctx.save_for_backward(pos, attr)
+            pix = max(c.renderer.total_pixels for c in renderer._chunks) if renderer.recompute else \
+                renderer.total_pixels
+            rast = torch.empty((pix, 4), dtype=torch.float32, device=pos.device)
+            words = torch.empty(pix, dtype=torch.int32, device=pos.device)
+            if renderer.recompute:
+                for c in renderer._chunks:
+                    c.renderer._forward_raw(pos[c.rows], attr, rast, None, out[c.floats], flags=words)
+            else:
+                renderer._forward_raw(pos, attr, rast, None, out, flags=words)
+            if keep:
+                ctx.save_for_backward(pos, attr)
             return out
         rast, color = renderer._buffers()
         out = torch.empty_like(color)
@@ -483,11 +498,11 @@ class _BatchFn(torch.autograd.Function):
                 cr._forward_raw(pos[c.rows], attr, rast, color, out, flags=flags)
                 cr._backward_raw(pos[c.rows], attr, rast, color, grad_out[c.floats], grad_pos[c.rows], grad_attr,
                                  cr._fwd_gen, aa_flags=flags)
-            return grad_pos, grad_attr, None
+            return grad_pos, grad_attr, None, None
         pos, attr, flags, rast, color = ctx.saved_tensors
         grad_pos, grad_attr = _zero_grads(pos, attr)
         r._backward_raw(pos, attr, rast, color, grad_out, grad_pos, grad_attr, ctx.gen, aa_flags=flags)
-        return grad_pos, grad_attr, None
+        return grad_pos, grad_attr, None, None
 
 
 class _BatchL1Fn(torch.autograd.Function):

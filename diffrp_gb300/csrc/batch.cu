@@ -34,6 +34,7 @@ struct BatchArgs {
     const int2* pix_blocks;   // (item, local block) per 256 pixels
     long long n_pix_blocks;
     long long total_prims, total_tiles;
+    long long total_pixels;  // drp_batch_render
     const float* pos;
     const int* tri;
     const float* attr;
@@ -49,7 +50,7 @@ struct BatchArgs {
     unsigned char* aa_flags;
     int* aa_list;
     unsigned* aa_count;
-    bool fit;               // the gradient-forming loss pass is batch_fit_kernel
+    bool fit;               // the fine raster writes the pixel words, for batch_fit_kernel or batch_blend_kernel
     uint32_t* aa_words;     // per pixel: triangle + 1 (0: none), kPixSil where its record has a silhouette edge
     bool emit_color;        // fit: the fine raster writes the colour of every pixel
     bool emit_out;          // the fine raster also writes the colour into out
@@ -448,6 +449,10 @@ constexpr long long kFitPixels = 1ll << 20;
 // nothing).  Region i leaves its |error| sum in a tile word the raster has
 // spent: the tile's list offset, or for the second half its cursor.
 __host__ __device__ inline int fit_regions_per_tile(int tile_log2) { return tile_log2 == 5 ? 2 : 1; }
+
+__device__ __forceinline__ bool fit_region_owner(int tile_log2, int tx, int ty) {
+    return tile_log2 == 5 || (tile_log2 == 4 ? (tx & 1) == 0 : (tx & 3) == 0 && (ty & 1) == 0);
+}
 
 __device__ __forceinline__ float* fit_loss_slot(const BatchArgs& a, long long i) {
     if (a.tile_log2 != 5) return reinterpret_cast<float*>(a.tile_offset + i);
@@ -857,20 +862,22 @@ constexpr int kFitRow = 44;
 constexpr int kFitStages = 3;  // rows of a walk in flight or in use
 
 // One warp's shared memory: the pair terms first, then the walk.
+template <int ROWS>
 struct FitPairsShared {
-    uint32_t words[10][36];       // the rows' words with one pixel around them (column 1 + lane)
-    unsigned short queue[8 * 72];  // pairs to evaluate: lane | row << 5 | slot << 8
-    float wt[8][32][4];           // weight of a pixel's slot
-    uint32_t flags[8][32];        // slots that blend | slots that blend into the pixel << 4
-    unsigned short blend[256];    // blended pixels: lane | row << 5
+    uint32_t words[ROWS + 2][36];           // the rows' words with one pixel around them (column 1 + lane)
+    unsigned short queue[32 * (2 * ROWS + 2)];  // pairs to evaluate: lane | row << 5 | slot << 8
+    float wt[ROWS][32][4];                  // weight of a pixel's slot
+    uint32_t flags[ROWS][32];               // slots that blend | slots that blend into the pixel << 4
+    unsigned short blend[32 * ROWS];        // blended pixels: lane | row << 5
 };
 struct FitWalkShared {
     float rows[32][kFitRow];
     float4 rast[kFitStages][32];       // the walk's rows: rast and
     float4 target[kFitStages][2][32];  // target (groups of four channels)
 };
+template <int ROWS>
 union FitShared {
-    FitPairsShared p;
+    FitPairsShared<ROWS> p;
     FitWalkShared w;
 };
 
@@ -950,9 +957,11 @@ __device__ __forceinline__ int warp_prefix(int v) {
 // place, a row with one such pair would run its chain of dependent loads
 // (depths, record, edge functions) for that lane alone.  The blended pixels are
 // then done one lane per (pixel, group of four channels), and the listed ones
-// take their places in the list with one atomic.
-template <bool VEC, int ROWS>
-__device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item& it, FitPairsShared& sh, int x0,
+// take their places in the list with one atomic.  LOSS = false (rendering):
+// the blended pixels' output only, no list and no error.
+template <bool VEC, int ROWS, bool LOSS>
+__device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item& it, FitPairsShared<ROWS>& sh,
+                                        int x0,
                                         int y0, int y1, FitClass& cl) {
     const int lane = threadIdx.x & 31, x = x0 + lane;
     const int W = it.width, H = it.height, C = it.channels;
@@ -1037,18 +1046,20 @@ __device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             const uint32_t f = sh.flags[r][lane];
-            if (f & 15u) cl.listed |= 1u << r;
+            if (LOSS && (f & 15u)) cl.listed |= 1u << r;
             if (f >> 4) blended |= 1u << r;
         }
         cl.live &= ~cl.listed;
         cl.plain &= ~blended;
         // listed pixels
-        const int lend = warp_prefix(__popc(cl.listed));
-        unsigned base = 0u;
-        if (lane == 31 && lend) base = atomicAdd(a.aa_count, (unsigned)lend);
-        base = __shfl_sync(0xffffffffu, base, 31) + (unsigned)(lend - __popc(cl.listed));
-        for (unsigned m = cl.listed; m; m &= m - 1)
-            a.aa_list[base++] = (int)(it.pixel_offset + p0 + (__ffs(m) - 1) * W);
+        if (LOSS) {
+            const int lend = warp_prefix(__popc(cl.listed));
+            unsigned base = 0u;
+            if (lane == 31 && lend) base = atomicAdd(a.aa_count, (unsigned)lend);
+            base = __shfl_sync(0xffffffffu, base, 31) + (unsigned)(lend - __popc(cl.listed));
+            for (unsigned m = cl.listed; m; m &= m - 1)
+                a.aa_list[base++] = (int)(it.pixel_offset + p0 + (__ffs(m) - 1) * W);
+        }
         // blended pixels
         const int bend = warp_prefix(__popc(blended)), nb = __shfl_sync(0xffffffffu, bend, 31);
         {
@@ -1065,7 +1076,7 @@ __device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item
             int slots = (int)(sh.flags[r][l] >> 4);
             const long long prow = it.image_offset + (long long)p * C + cg;
             float tg[4], y[3][4], base4[4], sv[4], val[4];
-            load4<VEC>(a.target + prow, C - cg, tg);
+            if (LOSS) load4<VEC>(a.target + prow, C - cg, tg);
             // the pixel and its sources in slot order (one as a rule): each
             // source's gathers are issued beside the ones before it
             auto vertices = [&](int sp, uint32_t word, float4& rp, int& t, int& j0, int& j1, int& j2) {
@@ -1103,7 +1114,7 @@ __device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item
             store4<VEC>(a.out + prow, C - cg, val);
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-                if (VEC || cg + c < C) sum += fabsf(val[c] - tg[c]);
+                if (LOSS && (VEC || cg + c < C)) sum += fabsf(val[c] - tg[c]);
         }
     }
     if (C > 32) cl.live = 0u;
@@ -1407,11 +1418,41 @@ __device__ __forceinline__ float fit_rows(const BatchArgs& a, const drp_batch_it
     return s;
 }
 
+// Rendering: blends the pixels that a pair touches into the image the fine
+// raster wrote.  One warp per 32 x ROWS pixels, on its own: most warps read
+// their words and are done.  What bounds it: the chain of dependent loads of
+// the pairs that blend (rows per warp: kBlendTallPixels).  Against one thread
+// per pixel testing the four pairs of its rast rows, with the colours kept
+// apart from the images so that a pair reads unblended ones: 84 instead of
+// 162 us for 5.8M pixels of ten meshes, and the fine raster, which then writes
+// one image instead of two, 443 instead of 619 us.
+constexpr int kBlendWarps = 4;
+template <int ROWS>
+__global__ void __launch_bounds__(32 * kBlendWarps) batch_blend_kernel(const __grid_constant__ BatchArgs a) {
+    __shared__ FitPairsShared<ROWS> sh[kBlendWarps];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, per_tile = 16 / ROWS * fit_regions_per_tile(a.tile_log2);
+    const long long unit = (long long)blockIdx.x * kBlendWarps + warp, tile_id = unit / per_tile;
+    if (tile_id >= a.total_tiles) return;
+    const drp_batch_item& it = a.items[find_item_by_tile(a.items, a.num_items, tile_id)];
+    const int tile = (int)(tile_id - it.tile_offset);
+    const int ty = tile / it.tiles_x, tx = tile - ty * it.tiles_x;
+    if (!fit_region_owner(a.tile_log2, tx, ty)) return;
+    const int y0 = (ty << a.tile_log2) + (int)(unit % per_tile) * ROWS, y1 = min(y0 + ROWS, it.height);
+    if (y0 >= y1) return;
+    const bool vec = (it.channels & 3) == 0 && ((reinterpret_cast<uintptr_t>(a.attr + it.attr_offset) |
+                                                 reinterpret_cast<uintptr_t>(a.out + it.image_offset)) & 15) == 0;
+    FitClass cl;
+    if (vec) fit_pairs<true, ROWS, false>(a, it, sh[warp], tx << a.tile_log2, y0, y1, cl);
+    else fit_pairs<false, ROWS, false>(a, it, sh[warp], tx << a.tile_log2, y0, y1, cl);
+}
+
 // One region of 32 x 16 pixels per CTA: WARPS warps of 16 / WARPS rows.
 template <int WARPS>
 __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) batch_fit_kernel(const __grid_constant__ BatchArgs a) {
     constexpr int ROWS = 16 / WARPS;
-    __shared__ __align__(16) FitShared sh[WARPS];
+    __shared__ __align__(16) FitShared<ROWS> sh[WARPS];
     __shared__ float warp_sum[WARPS];
     pdl_wait();
     pdl_launch_dependents();
@@ -1420,7 +1461,7 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) batch_fit_kernel(const
     const drp_batch_item& it = a.items[find_item_by_tile(a.items, a.num_items, tile_id)];
     const int tile = (int)(tile_id - it.tile_offset);
     const int ty = tile / it.tiles_x, tx = tile - ty * it.tiles_x;
-    const bool owner = a.tile_log2 == 5 || (a.tile_log2 == 4 ? (tx & 1) == 0 : (tx & 3) == 0 && (ty & 1) == 0);
+    const bool owner = fit_region_owner(a.tile_log2, tx, ty);
     const int warp = threadIdx.x >> 5;
     const int x0 = tx << a.tile_log2;
     const int y0 = (ty << a.tile_log2) + (int)(blockIdx.x % per_tile) * 16 + ROWS * warp;
@@ -1434,8 +1475,8 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) batch_fit_kernel(const
                            reinterpret_cast<uintptr_t>(a.out + it.image_offset) |
                            reinterpret_cast<uintptr_t>(a.color + it.image_offset)) & 15) == 0;
         FitClass cl;
-        if (vec) s = fit_pairs<true, ROWS>(a, it, sh[warp].p, x0, y0, y1, cl);
-        else s = fit_pairs<false, ROWS>(a, it, sh[warp].p, x0, y0, y1, cl);
+        if (vec) s = fit_pairs<true, ROWS, true>(a, it, sh[warp].p, x0, y0, y1, cl);
+        else s = fit_pairs<false, ROWS, true>(a, it, sh[warp].p, x0, y0, y1, cl);
         __syncwarp();  // the pair terms' shared memory becomes the walk's
         // walks hold the sums of four or eight channels; see fit_rows
         if (vec && it.channels == 8) s += fit_walk<2, true>(a, it, sh[warp].w, x0, y0, y1, cl);
@@ -1715,6 +1756,13 @@ static void carve(BatchArgs& a, void* ws, const BatchLayout& L) {
 // 64 views of 512 x 512, 32768 regions: 1039 against 946 us).
 constexpr long long kFitTallRegions = 4096;
 
+// Rows per warp of batch_blend_kernel: four read fewer words twice, but below
+// this many pixels two finish sooner -- the longest chain is that of the warp
+// with the most blends (344,438 pixels of small dense meshes: 217 with two,
+// 224 with four, 238 us with eight; 565,312: 157, 163, 174; 1,991,582: 422,
+// 420, 430; 5,848,746: 618, 591, 608).
+constexpr long long kBlendTallPixels = 1ll << 20;
+
 // Up to this many tiles per resident fine CTA the work order is sorted.
 constexpr long long kOrderTilesPerCTA = 8;
 
@@ -1850,6 +1898,14 @@ static bool side_stream(cudaStream_t s, SideStream& out) {
     return true;
 }
 
+template <int ROWS>
+static void launch_blend(const BatchArgs& a, long long regions, cudaStream_t s) {
+    const long long units = 16 / ROWS * regions;
+    launch_pdl(batch_blend_kernel<ROWS>, dim3((unsigned)((units + kBlendWarps - 1) / kBlendWarps)),
+               dim3(32 * kBlendWarps), s, a);
+    drp_note_launch();
+}
+
 int launch_batch_forward(BatchArgs a, void* ws, const BatchLayout& L, cudaStream_t s) {
     carve(a, ws, L);
     {
@@ -1903,6 +1959,14 @@ int launch_batch_forward(BatchArgs a, void* ws, const BatchLayout& L, cudaStream
             drp_note_launch();
         }
         launch_l1_final(a.block_loss, a.n_pix_blocks, a.l1_scale, a.loss, s);
+        return 0;
+    }
+    if (a.fit) {
+        if (a.n_pix_blocks > 0) {
+            const long long regions = a.total_tiles * fit_regions_per_tile(a.tile_log2);
+            if (a.total_pixels < kBlendTallPixels) launch_blend<2>(a, regions, s);
+            else launch_blend<4>(a, regions, s);
+        }
         return 0;
     }
     if (!a.out) return 0;  // raster + interpolation only (recomputing them for the backward)
@@ -2090,6 +2154,42 @@ DRP_API int drp_batch_forward(void* workspace, size_t workspace_bytes, const drp
     a.aa_records = out != nullptr;  // raster only: no antialias pass, no records
     drp::launch_batch_forward(a, workspace, L, static_cast<cudaStream_t>(stream));
     return drp_check_launch("drp_batch_forward");
+}
+
+DRP_API int drp_batch_render(void* workspace, size_t workspace_bytes, const drp_batch_item* items, int num_items,
+                             const int* prim_block_map, long long prim_blocks, const int* pixel_block_map,
+                             long long pixel_blocks, long long total_prims, long long total_tiles, const float* pos,
+                             const int* tri, const float* attr, const int* nbr, int tile_log2, int threads_per_tri,
+                             unsigned long long list_capacity, unsigned bin_depth, float* rast, void* words,
+                             float* out, long long total_pixels, void* stream) {
+    drp::BatchArgs a;
+    drp::BatchLayout L;
+    int st = batch_common(workspace, workspace_bytes, items, num_items, prim_block_map, prim_blocks, pixel_block_map,
+                          pixel_blocks, total_prims, total_tiles, list_capacity, pos, tri, attr, a, L);
+    if (st) return st;
+    if (tile_log2 < 3 || tile_log2 > 5) return bfail("batch: tile_log2 must be 3, 4 or 5");
+    if (threads_per_tri < 0 || threads_per_tri > 32 || (threads_per_tri & (threads_per_tri - 1)))
+        return bfail("batch: threads_per_tri must be 0 or a power of two <= 32");
+    if (!rast || !words || !out || total_pixels <= 0 || (reinterpret_cast<uintptr_t>(rast) & 15) ||
+        (reinterpret_cast<uintptr_t>(words) & 3))
+        return bfail("batch: bad outputs");
+    if (bin_depth && (unsigned long long)total_tiles * bin_depth > list_capacity)
+        return bfail("batch: list_capacity below total_tiles * bin_depth");
+    a.nbr = nbr;
+    a.tile_log2 = tile_log2;
+    a.tpt = threads_per_tri;
+    a.bin_depth = bin_depth;
+    a.rast = rast;
+    a.color = out;  // the fine raster writes the colours in place
+    a.out = out;
+    a.aa_words = static_cast<uint32_t*>(words);
+    a.total_pixels = total_pixels;
+    a.fit = true;
+    a.emit_color = true;
+    a.emit_out = false;
+    a.aa_records = true;
+    drp::launch_batch_forward(a, workspace, L, static_cast<cudaStream_t>(stream));
+    return drp_check_launch("drp_batch_render");
 }
 
 DRP_API int drp_batch_forward_l1(void* workspace, size_t workspace_bytes, const drp_batch_item* items, int num_items,

@@ -152,6 +152,7 @@ DRP_FAST(drp_transform_points_fwd)
 DRP_FAST(drp_transform_points_bwd)
 DRP_FAST(drp_copy_async)
 DRP_FAST(drp_batch_forward)
+DRP_FAST(drp_batch_render)
 DRP_FAST(drp_batch_forward_l1)
 DRP_FAST(drp_batch_forward_l1_grad)
 DRP_FAST(drp_batch_fit_l1)
@@ -178,6 +179,7 @@ PyMethodDef methods[] = {
     DRP_ENTRY(drp_transform_points_bwd),
     DRP_ENTRY(drp_copy_async),
     DRP_ENTRY(drp_batch_forward),
+    DRP_ENTRY(drp_batch_render),
     DRP_ENTRY(drp_batch_forward_l1),
     DRP_ENTRY(drp_batch_forward_l1_grad),
     DRP_ENTRY(drp_batch_fit_l1),

@@ -414,6 +414,21 @@ int drp_batch_forward(void* workspace, size_t workspace_bytes, const drp_batch_i
                       unsigned long long list_capacity, unsigned bin_depth, float* rast, float* color, float* out,
                       void* aa_state, long long total_pixels, void* stream);
 
+/*
+ * drp_batch_forward for a caller that wants the images alone and no backward:
+ * out is the only image written (the colours in place, then the blended
+ * pixels).  rast and words (one 32-bit word per pixel: its triangle, and
+ * whether that has a silhouette edge) are scratch of total_pixels rows / words.
+ * The images equal drp_batch_forward's bit for bit.  No counterpart in the
+ * reference.
+ */
+int drp_batch_render(void* workspace, size_t workspace_bytes, const drp_batch_item* items, int num_items,
+                     const int* prim_block_map, long long prim_blocks, const int* pixel_block_map,
+                     long long pixel_blocks, long long total_prims, long long total_tiles, const float* pos,
+                     const int* tri, const float* attr, const int* nbr, int tile_log2, int threads_per_tri,
+                     unsigned long long list_capacity, unsigned bin_depth, float* rast, void* words, float* out,
+                     long long total_pixels, void* stream);
+
 /* Bytes of the antialias state block of drp_batch_forward (total_pixels =
  * totals[2] of drp_batch_plan). */
 int drp_batch_aa_state_size(long long total_pixels, size_t* bytes);
