@@ -186,6 +186,18 @@ __device__ __forceinline__ void copy_channels(const float* src, float* dst, int 
     }
 }
 
+// Four channels of an image row: one vector (VEC) or the n below four.
+template <bool VEC>
+__device__ __forceinline__ void load_channels(const float* p, int n, float (&x)[4]) {
+    if (VEC) {
+        const float4 q = *reinterpret_cast<const float4*>(p);
+        x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = k < n ? p[k] : 0.f;
+    }
+}
+
 // Blend terms of one pixel: for each pair slot (left, right, below, above)
 // whose pair blends into this pixel, the source pixel and its weight.  The
 // pixel's and its four neighbours' rast rows are loaded together, before any
@@ -284,8 +296,7 @@ __device__ __forceinline__ bool aa_fwd_terms_row(const float4* R, const float4* 
     return any;
 }
 
-// A pixel's word as the batched fine raster writes it: its triangle + 1 (0:
-// background) and kPixSil when that triangle's antialias record has a
+// A pixel's word: its triangle + 1 (0: background) and kPixSil when that triangle's antialias record has a
 // silhouette edge.  A pair whose front triangle has none never blends
 // (aa_pair), so two unequal ids without the bit need no record and no rast
 // row: inside a closed mesh that is almost every pair.
@@ -293,6 +304,114 @@ constexpr uint32_t kPixSil = 0x80000000u;
 
 __device__ __forceinline__ bool pix_pair_may_blend(uint32_t a, uint32_t b) {
     return ((a ^ b) & ~kPixSil) != 0u && ((a | b) & kPixSil) != 0u;
+}
+
+// ---------------------------------------------------------------------------
+// Pair terms by warps: 32 columns x ROWS rows, one column per lane.
+// ---------------------------------------------------------------------------
+template <int ROWS>
+struct PairShared {
+    uint32_t words[ROWS + 2][36];           // the rows' words with one pixel around them (column 1 + lane)
+    unsigned short queue[32 * (2 * ROWS + 2)];  // pairs to evaluate: lane | row << 5 | slot << 8
+    float wt[ROWS][32][4];                  // weight of a pixel's slot
+    uint32_t flags[ROWS][32];               // slots that blend | slots that blend into the pixel << 4
+    unsigned short blend[32 * ROWS];        // blended pixels: lane | row << 5
+};
+// Inclusive prefix sum over the warp.
+__device__ __forceinline__ int warp_prefix(int v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += y;
+    }
+    return v;
+}
+
+// The pairs of the rows [y0, y1) (at most ROWS) x columns [x0, x0 + 32) of one
+// image, by one warp.  w[1 + r]: the lane's pixel word of row y0 + r, w[0] and
+// the one after the last row: its lower and upper neighbours' (0 outside the
+// image); side[r]: the word left of lane 0's and right of lane 31's pixel.  The
+// words decide which pairs may blend (the row's right neighbours and the upper
+// ones; at the region's left and lower border the outer pairs too, so a pair
+// inside is evaluated once); those go through a queue, so that 32 lanes evaluate
+// 32 pairs -- left in place, a row with one such pair would run its chain of
+// dependent loads (depths, record, edge functions) for that lane alone.
+// listed / blended (one bit per row): the lane's pixels that some pair touches /
+// that one blends into; sh.flags[r][lane]: which slots, sh.wt[r][lane][slot]
+// their weights, sh.words[r + 1][1 + lane] the words.  Returns false (warp
+// uniform) when no pair may blend; nothing in sh is written then.
+// depth(pixel, column - x0, row - y0): a pixel's depth; rec: the image's triangle
+// records.  All 32 lanes call it (it synchronises the warp before any depth).
+template <int ROWS, class Depth>
+__device__ __forceinline__ bool warp_pairs(const Depth& depth, const float4* rec, int W, int H, int x0, int y0, int y1,
+                                           const uint32_t (&w)[ROWS + 2], const uint32_t (&side)[ROWS],
+                                           PairShared<ROWS>& sh, unsigned& listed, unsigned& blended) {
+    const int lane = threadIdx.x & 31, x = x0 + lane;
+    const bool in = x < W, has_left = lane == 0 && x > 0;
+    unsigned need = 0u;  // four bits per row
+    listed = blended = 0u;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        uint32_t nb = __shfl_down_sync(0xffffffffu, w[r + 1], 1);
+        if (lane == 31) nb = side[r];
+        const int y = y0 + r;
+        if (!in || y >= y1) continue;
+        if (x + 1 < W && pix_pair_may_blend(w[r + 1], nb)) need |= 2u << (4 * r);
+        if (y + 1 < H && pix_pair_may_blend(w[r + 1], w[r + 2])) need |= 8u << (4 * r);
+        if (has_left && pix_pair_may_blend(w[r + 1], side[r])) need |= 1u << (4 * r);
+        if (r == 0 && y > 0 && pix_pair_may_blend(w[1], w[0])) need |= 4u;
+    }
+    const int last = warp_prefix(__popc(need)), total = __shfl_sync(0xffffffffu, last, 31);
+    if (!total) return false;
+    {
+        int e = last - __popc(need);
+        for (unsigned m = need; m; m &= m - 1) {
+            const int b = __ffs(m) - 1;
+            sh.queue[e++] = (unsigned short)(lane | ((b >> 2) << 5) | ((b & 3) << 8));
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS + 2; ++r) sh.words[r][1 + lane] = w[r];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        sh.flags[r][lane] = 0u;
+        if (lane == 0) sh.words[r + 1][0] = side[r];
+        if (lane == 31) sh.words[r + 1][33] = side[r];
+    }
+    __syncwarp();
+    for (int k = lane; k < total; k += 32) {
+        const int e = sh.queue[k], l = e & 31, r = (e >> 5) & 7, q = e >> 8;
+        const int dx = q == 0 ? -1 : (q == 1 ? 1 : 0), dy = q == 2 ? -1 : (q == 3 ? 1 : 0);
+        const int px = x0 + l, py = y0 + r, pix = py * W + px;
+        const float zs = depth(pix, l, r), zn = depth(pix + dx + dy * W, l + dx, r + dy);
+        const int t = (int)(sh.words[r + 1][l + 1] & ~kPixSil) - 1;
+        const int tn = (int)(sh.words[r + 1 + dy][l + 1 + dx] & ~kPixSil) - 1;
+        // the front pixel as aa_pair chooses it: the nearer one, or the
+        // only covered one; equal depths: the lower triangle
+        const bool self_front = tn < 0 || (t >= 0 && (zs < zn || (!(zn < zs) && t < tn)));
+        int A_, B_, ax, ay;
+        bool vert;
+        pair_slot(q, pix, px, py, W, H, A_, B_, ax, ay, vert);
+        AAPair pr;
+        aa_pair_edges(rec, self_front ? t : tn, self_front == (A_ == pix), A_, B_, ax, ay, vert, pr);
+        if (!pr.valid) continue;
+        const bool mine = pr.target == pix;
+        atomicOr(&sh.flags[r][l], (mine ? 17u : 1u) << q);
+        sh.wt[r][l][q] = pr.w;
+        if ((q == 1 && l < 31) || (q == 3 && py + 1 < y1)) {  // the neighbour is this warp's too: its opposite slot
+            atomicOr(&sh.flags[r + dy][l + dx], (mine ? 1u : 17u) << (q - 1));
+            sh.wt[r + dy][l + dx][q - 1] = pr.w;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        const uint32_t f = sh.flags[r][lane];
+        if (f & 15u) listed |= 1u << r;
+        if (f >> 4) blended |= 1u << r;
+    }
+    return true;
 }
 
 // Forward of one pixel: out = c + sum over pair slots targeting this pixel of

@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(256) aa_setup_kernel(AAArgs a) {
     aa_tri_record(P, a.tri, a.nbr, t, a.num_triangles, a.num_vertices, a.W, a.H, rec);
 }
 
+// Forward of small launches (kFwdRegionPixels): one thread per pixel.
 __global__ void __launch_bounds__(256) aa_fwd_kernel(AAArgs a) {
     const int b = blockIdx.y;
     const int npix = a.H * a.W;
@@ -154,6 +155,149 @@ __global__ void __launch_bounds__(256) aa_fwd_kernel(AAArgs a) {
     if (lane == leader) base = atomicAdd(a.list_count, (unsigned)__popc(m));
     base = __shfl_sync(0xffffffffu, base, leader);
     if (need) a.list[base + __popc(m & ((1u << lane) - 1u))] = b * npix + pix;
+}
+
+// Forward of larger launches: one warp per 32 columns x kFwdRows rows of a view.  It copies its
+// pixels' colours, makes their words (triangle, silhouette bit) from the rast
+// rows and the records, and blends where warp_pairs finds a pair that does; a
+// blended pixel is then written again, one lane per (pixel, four channels).
+// What bounds it: the traffic (rast once, colours in and out) and, on a view
+// full of silhouettes, the pairs.  Six views of 800 x 1000 x 8 channels: 84
+// instead of 140 us (4.6 TB/s); eight of 512 x 512 x 3: 34 instead of 67.  Four
+// rows per warp measured the same, one row 121 and 49.
+constexpr int kFwdWarps = 4, kFwdRows = 2;
+
+struct FwdShared {
+    PairShared<kFwdRows> p;
+    float depth[kFwdRows + 2][36];  // as p.words
+};
+
+__device__ __forceinline__ float2 depth_id(const float4* r) { return reinterpret_cast<const float2*>(r)[1]; }
+
+template <bool VEC>
+__device__ __forceinline__ void aa_fwd_region(const AAArgs& a, int b, int x0, int y0, FwdShared& sh) {
+    const int lane = threadIdx.x & 31, x = x0 + lane;
+    const int W = a.W, H = a.H, C = a.C, npix = H * W;
+    const int y1 = min(y0 + kFwdRows, H), cols = min(32, W - x0);
+    const float4* R = reinterpret_cast<const float4*>(a.rast) + (long long)b * npix;
+    const float4* rec = reinterpret_cast<const float4*>(a.tri_rec) + (long long)b * a.num_triangles * 2;
+    const float* src = a.color + (long long)b * npix * C;
+    float* dst = a.out + (long long)b * npix * C;
+    const bool in = x < W;
+    const int p0 = y0 * W + x;
+    // the ids first: the copy fills the time of their loads
+    float2 id[kFwdRows + 2], idside[kFwdRows];  // depth, triangle
+    const bool edge = (lane == 0 && x > 0) || (lane == 31 && x + 1 < W);
+#pragma unroll
+    for (int r = 0; r < kFwdRows + 2; ++r) {
+        const int y = y0 - 1 + r;
+        id[r] = in && y >= 0 && y < H && y <= y1 ? depth_id(R + p0 + (r - 1) * W) : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int r = 0; r < kFwdRows; ++r)
+        idside[r] = y0 + r < y1 && edge ? depth_id(R + p0 + r * W + (lane == 0 ? -1 : 1)) : make_float2(0.f, 0.f);
+    {
+        // all rows of a column group are loaded before the first is stored
+        const long long row = (long long)(y0 * W + x0) * C, step = (long long)W * C;
+        const int n = cols * C;
+        if (a.copy4) {
+            const float4* s4 = reinterpret_cast<const float4*>(src + row);
+            float4* d4 = reinterpret_cast<float4*>(dst + row);
+            const long long step4 = step >> 2;
+            for (int k = lane; k < n >> 2; k += 32) {
+                float4 v[kFwdRows];
+#pragma unroll
+                for (int r = 0; r < kFwdRows; ++r)
+                    if (y0 + r < y1) v[r] = s4[r * step4 + k];
+#pragma unroll
+                for (int r = 0; r < kFwdRows; ++r)
+                    if (y0 + r < y1) d4[r * step4 + k] = v[r];
+            }
+        } else {
+            for (int k = lane; k < n; k += 32) {
+                float v[kFwdRows];
+#pragma unroll
+                for (int r = 0; r < kFwdRows; ++r)
+                    if (y0 + r < y1) v[r] = src[row + r * step + k];
+#pragma unroll
+                for (int r = 0; r < kFwdRows; ++r)
+                    if (y0 + r < y1) dst[row + r * step + k] = v[r];
+            }
+        }
+    }
+    const auto word = [&](float f) {
+        const int t = rast_tri(f);
+        if (t < 0 || t >= a.num_triangles) return 0u;
+        return (uint32_t)(t + 1) | (__float_as_uint(rec[2 * (long long)t + 1].w) ? kPixSil : 0u);
+    };
+    uint32_t w[kFwdRows + 2], side[kFwdRows];
+#pragma unroll
+    for (int r = 0; r < kFwdRows + 2; ++r) w[r] = word(id[r].y);
+#pragma unroll
+    for (int r = 0; r < kFwdRows; ++r) side[r] = word(idside[r].y);
+#pragma unroll
+    for (int r = 0; r < kFwdRows + 2; ++r) sh.depth[r][1 + lane] = id[r].x;
+#pragma unroll
+    for (int r = 0; r < kFwdRows; ++r) {
+        if (lane == 0) sh.depth[r + 1][0] = idside[r].x;
+        if (lane == 31) sh.depth[r + 1][33] = idside[r].x;
+    }
+    const auto depth = [&](int, int l, int row) { return sh.depth[1 + row][1 + l]; };
+    unsigned listed, blended;
+    if (!warp_pairs<kFwdRows>(depth, rec, W, H, x0, y0, y1, w, side, sh.p, listed, blended)) return;
+    if (a.list) {
+        const int end = warp_prefix(__popc(listed));
+        unsigned base = 0u;
+        if (lane == 31 && end) base = atomicAdd(a.list_count, (unsigned)end);
+        base = __shfl_sync(0xffffffffu, base, 31) + (unsigned)(end - __popc(listed));
+        for (unsigned m = listed; m; m &= m - 1) a.list[base++] = b * npix + p0 + (__ffs(m) - 1) * W;
+    }
+    const int bend = warp_prefix(__popc(blended)), nb = __shfl_sync(0xffffffffu, bend, 31);
+    {
+        int e = bend - __popc(blended);
+        for (unsigned m = blended; m; m &= m - 1) sh.p.blend[e++] = (unsigned short)(lane | ((__ffs(m) - 1) << 5));
+    }
+    __syncwarp();  // the list of blends, and the copied colours they replace
+    const int per = (C + 3) >> 2, tasks = nb * per;
+#pragma unroll 1
+    for (int k = lane; k < tasks; k += 32) {
+        const int e = k / per, cg = 4 * (k - e * per);
+        const int l = sh.p.blend[e] & 31, r = sh.p.blend[e] >> 5, n = C - cg;
+        const int p = (y0 + r) * W + x0 + l;
+        float base4[4], sv[4], val[4];
+        load_channels<VEC>(src + (long long)p * C + cg, n, base4);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) val[c] = base4[c];
+        for (int slots = (int)(sh.p.flags[r][l] >> 4); slots; slots &= slots - 1) {  // in slot order
+            const int q = __ffs(slots) - 1;
+            const int sp = p + (q == 0 ? -1 : (q == 1 ? 1 : (q == 2 ? -W : W)));
+            load_channels<VEC>(src + (long long)sp * C + cg, n, sv);
+            const float wq = sh.p.wt[r][l][q];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) val[c] = fmaf(wq, sv[c] - base4[c], val[c]);
+        }
+        float* o = dst + (long long)p * C + cg;
+        if (VEC) {
+            *reinterpret_cast<float4*>(o) = make_float4(val[0], val[1], val[2], val[3]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (c < n) o[c] = val[c];
+        }
+    }
+}
+
+__global__ void __launch_bounds__(32 * kFwdWarps) aa_fwd_region_kernel(AAArgs a, int units_x, int units_y) {
+    __shared__ FwdShared sh[kFwdWarps];
+    const int warp = threadIdx.x >> 5;
+    const long long unit = (long long)blockIdx.x * kFwdWarps + warp;
+    const long long row = unit / units_x;
+    const int b = (int)(row / units_y);
+    if (b >= a.B) return;
+    const int x0 = 32 * (int)(unit - row * units_x), y0 = kFwdRows * (int)(row - (long long)b * units_y);
+    const bool vec = (a.C & 3) == 0 && (((uintptr_t)a.color | (uintptr_t)a.out) & 15) == 0;
+    if (vec) aa_fwd_region<true>(a, b, x0, y0, sh[warp]);
+    else aa_fwd_region<false>(a, b, x0, y0, sh[warp]);
 }
 
 // With the forward's pixel list the colour gradient is the incoming one
@@ -267,13 +411,28 @@ static void launch_aa_setup(const AAArgs& a, cudaStream_t s) {
     drp_note_launch();
 }
 
+// From this many pixels on the forward goes by regions.  Below, a warp's chain
+// of loads (ids, then records) is what counts: one 200 x 200 view of 3 channels
+// takes 21.3 us by regions of one row and 20.8 by pixels (forward and backward;
+// 27.6 and 26.2 with a mesh of 82k triangles), one of 512 x 512 22.8 and 25.0.
+constexpr long long kFwdRegionPixels = 1ll << 17;
+
 int launch_aa_fwd(const AAArgs& a, cudaStream_t s) {
     const int npix = a.H * a.W;
     if (npix == 0) return 0;
     if (a.list_count) cudaMemsetAsync(a.list_count, 0, sizeof(unsigned), s);
     launch_aa_setup(a, s);
-    dim3 grid((unsigned)((npix + 255) / 256), (unsigned)a.B);
-    aa_fwd_kernel<<<grid, 256, 0, s>>>(a);
+    if ((long long)a.B * npix < kFwdRegionPixels) {
+        dim3 grid((unsigned)((npix + 255) / 256), (unsigned)a.B);
+        aa_fwd_kernel<<<grid, 256, 0, s>>>(a);
+    } else {
+        AAArgs c = a;
+        // every row of every region starts on 16 bytes
+        c.copy4 = ((long long)a.W * a.C) % 4 == 0 && (((uintptr_t)a.color | (uintptr_t)a.out) & 15) == 0;
+        const int ux = (a.W + 31) / 32, uy = (a.H + kFwdRows - 1) / kFwdRows;
+        const long long units = (long long)a.B * ux * uy;
+        aa_fwd_region_kernel<<<(unsigned)((units + kFwdWarps - 1) / kFwdWarps), 32 * kFwdWarps, 0, s>>>(c, ux, uy);
+    }
     drp_note_launch();
     return 0;
 }

@@ -806,18 +806,7 @@ __device__ __forceinline__ float l1_sign_fast(float d, float scale) {
     return g;
 }
 
-// Four channels of an image row: one vector (VEC) or the channels below C.
-template <bool VEC>
-__device__ __forceinline__ void load4(const float* p, int n, float (&x)[4]) {
-    if (VEC) {
-        const float4 q = *reinterpret_cast<const float4*>(p);
-        x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
-    } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) x[k] = k < n ? p[k] : 0.f;
-    }
-}
-
+// The same four written back (load_channels).
 template <bool VEC>
 __device__ __forceinline__ void store4(float* p, int n, const float (&x)[4]) {
     if (VEC) {
@@ -861,15 +850,7 @@ __device__ __forceinline__ void store4(float* p, int n, const float (&x)[4]) {
 constexpr int kFitRow = 44;
 constexpr int kFitStages = 3;  // rows of a walk in flight or in use
 
-// One warp's shared memory: the pair terms first, then the walk.
-template <int ROWS>
-struct FitPairsShared {
-    uint32_t words[ROWS + 2][36];           // the rows' words with one pixel around them (column 1 + lane)
-    unsigned short queue[32 * (2 * ROWS + 2)];  // pairs to evaluate: lane | row << 5 | slot << 8
-    float wt[ROWS][32][4];                  // weight of a pixel's slot
-    uint32_t flags[ROWS][32];               // slots that blend | slots that blend into the pixel << 4
-    unsigned short blend[32 * ROWS];        // blended pixels: lane | row << 5
-};
+// One warp's shared memory: the pair terms (PairShared) first, then the walk.
 struct FitWalkShared {
     float rows[32][kFitRow];
     float4 rast[kFitStages][32];       // the walk's rows: rast and
@@ -877,7 +858,7 @@ struct FitWalkShared {
 };
 template <int ROWS>
 union FitShared {
-    FitPairsShared<ROWS> p;
+    PairShared<ROWS> p;
     FitWalkShared w;
 };
 
@@ -937,32 +918,16 @@ struct FitClass {
     unsigned live, plain, listed;
 };
 
-// Inclusive prefix sum over the warp.
-__device__ __forceinline__ int warp_prefix(int v) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, v, d);
-        if (lane >= d) v += y;
-    }
-    return v;
-}
-
 // Pair terms of the rows [y0, y1) (at most ROWS) x columns [x0, x0 + 32) by one
-// warp, and with them everything of the pixels a pair blends into: their
-// output and |error| (returned, per lane).  The words decide which pairs may
-// blend (the row's right neighbours and the upper ones; at the region's left
-// and lower border the outer pairs too, so a pair inside is evaluated once);
-// those go through a queue, so that 32 lanes evaluate 32 pairs -- left in
-// place, a row with one such pair would run its chain of dependent loads
-// (depths, record, edge functions) for that lane alone.  The blended pixels are
-// then done one lane per (pixel, group of four channels), and the listed ones
-// take their places in the list with one atomic.  LOSS = false (rendering):
-// the blended pixels' output only, no list and no error.
+// warp (warp_pairs, from the words the fine raster wrote), and with them
+// everything of the pixels a pair blends into: their output and |error|
+// (returned, per lane).  The blended pixels are done one lane per (pixel, group
+// of four channels), and the listed ones take their places in the list with
+// one atomic.  LOSS = false (rendering): the blended pixels' output only, no
+// list and no error.
 template <bool VEC, int ROWS, bool LOSS>
-__device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item& it, FitPairsShared<ROWS>& sh,
-                                        int x0,
-                                        int y0, int y1, FitClass& cl) {
+__device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item& it, PairShared<ROWS>& sh,
+                                        int x0, int y0, int y1, FitClass& cl) {
     const int lane = threadIdx.x & 31, x = x0 + lane;
     const int W = it.width, H = it.height, C = it.channels;
     const bool in = x < W;
@@ -971,84 +936,27 @@ __device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item
     const int* tri = a.tri + 3 * (long long)it.tri_first;
     const float* A = a.attr + it.attr_offset;
     const int p0 = y0 * W + x;
-    const bool has_left = lane == 0 && x > 0, has_right = lane == 31 && x + 1 < W;
     uint32_t w[ROWS + 2], side[ROWS];  // rows y0 - 1 .. y1
 #pragma unroll
     for (int r = 0; r < ROWS + 2; ++r) {
         const int y = y0 - 1 + r;
         w[r] = in && y >= 0 && y < H && y <= y1 ? Wd[p0 + (r - 1) * W] : 0u;
     }
+    const bool edge = (lane == 0 && x > 0) || (lane == 31 && x + 1 < W);
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r)
-        side[r] = y0 + r < y1 && (has_left || has_right) ? Wd[p0 + r * W + (lane == 0 ? -1 : 1)] : 0u;
-    unsigned need = 0u;  // four bits per row
+    for (int r = 0; r < ROWS; ++r) side[r] = y0 + r < y1 && edge ? Wd[p0 + r * W + (lane == 0 ? -1 : 1)] : 0u;
     cl.live = cl.plain = cl.listed = 0u;
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
-        uint32_t nb = __shfl_down_sync(0xffffffffu, w[r + 1], 1);
-        if (lane == 31) nb = side[r];
-        const int y = y0 + r;
-        if (!in || y >= y1) continue;
+        if (!in || y0 + r >= y1) continue;
         cl.plain |= 1u << r;
         if (w[r + 1] & ~kPixSil) cl.live |= 1u << r;
-        if (x + 1 < W && pix_pair_may_blend(w[r + 1], nb)) need |= 2u << (4 * r);
-        if (y + 1 < H && pix_pair_may_blend(w[r + 1], w[r + 2])) need |= 8u << (4 * r);
-        if (has_left && pix_pair_may_blend(w[r + 1], side[r])) need |= 1u << (4 * r);
-        if (r == 0 && y > 0 && pix_pair_may_blend(w[1], w[0])) need |= 4u;
     }
     float sum = 0.f;
-    const int last = warp_prefix(__popc(need)), total = __shfl_sync(0xffffffffu, last, 31);
-    if (total) {
-        {
-            int e = last - __popc(need);
-            for (unsigned m = need; m; m &= m - 1) {
-                const int b = __ffs(m) - 1;
-                sh.queue[e++] = (unsigned short)(lane | ((b >> 2) << 5) | ((b & 3) << 8));
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < ROWS + 2; ++r) sh.words[r][1 + lane] = w[r];
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            sh.flags[r][lane] = 0u;
-            if (lane == 0) sh.words[r + 1][0] = side[r];
-            if (lane == 31) sh.words[r + 1][33] = side[r];
-        }
-        __syncwarp();
-        const float4* rec = a.aa_rec + it.prim_offset * 2;
-        for (int k = lane; k < total; k += 32) {
-            const int e = sh.queue[k], l = e & 31, r = (e >> 5) & 7, q = e >> 8;
-            const int dx = q == 0 ? -1 : (q == 1 ? 1 : 0), dy = q == 2 ? -1 : (q == 3 ? 1 : 0);
-            const int px = x0 + l, py = y0 + r, pix = py * W + px;
-            const float zs = reinterpret_cast<const float*>(R + pix)[2];
-            const float zn = reinterpret_cast<const float*>(R + pix + dx + dy * W)[2];
-            const int t = (int)(sh.words[r + 1][l + 1] & ~kPixSil) - 1;
-            const int tn = (int)(sh.words[r + 1 + dy][l + 1 + dx] & ~kPixSil) - 1;
-            // the front pixel as aa_pair chooses it: the nearer one, or the
-            // only covered one; equal depths: the lower triangle
-            const bool self_front = tn < 0 || (t >= 0 && (zs < zn || (!(zn < zs) && t < tn)));
-            int A_, B_, ax, ay;
-            bool vert;
-            pair_slot(q, pix, px, py, W, H, A_, B_, ax, ay, vert);
-            AAPair pr;
-            aa_pair_edges(rec, self_front ? t : tn, self_front == (A_ == pix), A_, B_, ax, ay, vert, pr);
-            if (!pr.valid) continue;
-            const bool mine = pr.target == pix;
-            atomicOr(&sh.flags[r][l], (mine ? 17u : 1u) << q);
-            sh.wt[r][l][q] = pr.w;
-            if ((q == 1 && l < 31) || (q == 3 && py + 1 < y1)) {  // the neighbour is this warp's too: its opposite slot
-                atomicOr(&sh.flags[r + dy][l + dx], (mine ? 1u : 17u) << (q - 1));
-                sh.wt[r + dy][l + dx][q - 1] = pr.w;
-            }
-        }
-        __syncwarp();
-        unsigned blended = 0u;
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            const uint32_t f = sh.flags[r][lane];
-            if (LOSS && (f & 15u)) cl.listed |= 1u << r;
-            if (f >> 4) blended |= 1u << r;
-        }
+    unsigned listed, blended;
+    const auto depth = [&](int pix, int, int) { return reinterpret_cast<const float*>(R + pix)[2]; };
+    if (warp_pairs<ROWS>(depth, a.aa_rec + it.prim_offset * 2, W, H, x0, y0, y1, w, side, sh, listed, blended)) {
+        if (LOSS) cl.listed = listed;
         cl.live &= ~cl.listed;
         cl.plain &= ~blended;
         // listed pixels
@@ -1076,7 +984,7 @@ __device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item
             int slots = (int)(sh.flags[r][l] >> 4);
             const long long prow = it.image_offset + (long long)p * C + cg;
             float tg[4], y[3][4], base4[4], sv[4], val[4];
-            if (LOSS) load4<VEC>(a.target + prow, C - cg, tg);
+            if (LOSS) load_channels<VEC>(a.target + prow, C - cg, tg);
             // the pixel and its sources in slot order (one as a rule): each
             // source's gathers are issued beside the ones before it
             auto vertices = [&](int sp, uint32_t word, float4& rp, int& t, int& j0, int& j1, int& j2) {
@@ -1354,8 +1262,8 @@ __device__ __forceinline__ float fit_rows(const BatchArgs& a, const drp_batch_it
         if (in) {
             t = (int)(Wd[pix] & ~kPixSil) - 1;
             r = R[pix];
-            load4<VEC>(a.target + row, C, tv[0]);
-            if (C > 4) load4<VEC>(a.target + row + 4, C - 4, tv[1]);
+            load_channels<VEC>(a.target + row, C, tv[0]);
+            if (C > 4) load_channels<VEC>(a.target + row + 4, C - 4, tv[1]);
             if (t >= 0) {
                 i0 = tri[3 * (long long)t];
                 i1 = tri[3 * (long long)t + 1];
@@ -1388,7 +1296,7 @@ __device__ __forceinline__ float fit_rows(const BatchArgs& a, const drp_batch_it
                 }
                 if (plain) store4<VEC>(a.out + row + cg, C - cg, val);
                 if (keep_color) store4<VEC>(a.color + row + cg, C - cg, val);
-                if (in && cg + 8 < C) load4<VEC>(a.target + row + cg + 8, C - cg - 8, tv[gi]);
+                if (in && cg + 8 < C) load_channels<VEC>(a.target + row + cg + 8, C - cg - 8, tv[gi]);
                 if (live) {
                     float4* d = reinterpret_cast<float4*>(rw + 12 * gi);
                     d[0] = make_float4(g[0] * u, g[1] * u, g[2] * u, g[3] * u);
@@ -1429,7 +1337,7 @@ __device__ __forceinline__ float fit_rows(const BatchArgs& a, const drp_batch_it
 constexpr int kBlendWarps = 4;
 template <int ROWS>
 __global__ void __launch_bounds__(32 * kBlendWarps) batch_blend_kernel(const __grid_constant__ BatchArgs a) {
-    __shared__ FitPairsShared<ROWS> sh[kBlendWarps];
+    __shared__ PairShared<ROWS> sh[kBlendWarps];
     pdl_wait();
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, per_tile = 16 / ROWS * fit_regions_per_tile(a.tile_log2);

@@ -134,6 +134,7 @@ struct AAArgs {
     // touches; the backward then evaluates the antialias terms of those only)
     unsigned* list_count;
     int* list;
+    bool copy4;  // forward: rows can be copied by 16 bytes
 };
 
 // Bytes of the drp_antialias_fwd / _bwd pixel-list state for B views of H x W.
