@@ -31,6 +31,8 @@ _SIGNATURES = {
     "drp_edge_gradient_bwd": [_P, _P, _LL, _P, _P, _I, _P, _I, _I, _P, _P],
     "drp_l1_loss_workspace_size": [_LL, _SZ],
     "drp_l1_loss_fwd": [_P, ctypes.c_size_t, _P, _P, _LL, _F, _P, _P, _P],
+    "drp_l1_loss_sign_fwd": [_P, ctypes.c_size_t, _P, _P, _LL, _F, _P, _P, _P],
+    "drp_l1_loss_bwd": [_P, _LL, _F, _P, _P, _P],
     "drp_transform_points_fwd": [_P, _LL, _P, ctypes.c_int, _P, _P],
     "drp_transform_points_bwd": [_P, _LL, _P, ctypes.c_int, _P, _P],
     "drp_host_device_pointer": [_P, _P],

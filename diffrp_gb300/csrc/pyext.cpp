@@ -145,6 +145,8 @@ DRP_FAST(drp_antialias_fwd)
 DRP_FAST(drp_antialias_bwd)
 DRP_FAST(drp_edge_gradient_bwd)
 DRP_FAST(drp_l1_loss_fwd)
+DRP_FAST(drp_l1_loss_sign_fwd)
+DRP_FAST(drp_l1_loss_bwd)
 DRP_FAST(drp_texture_mip_build)
 DRP_FAST(drp_texture_fwd)
 DRP_FAST(drp_texture_bwd)
@@ -172,6 +174,8 @@ PyMethodDef methods[] = {
     DRP_ENTRY(drp_antialias_bwd),
     DRP_ENTRY(drp_edge_gradient_bwd),
     DRP_ENTRY(drp_l1_loss_fwd),
+    DRP_ENTRY(drp_l1_loss_sign_fwd),
+    DRP_ENTRY(drp_l1_loss_bwd),
     DRP_ENTRY(drp_texture_mip_build),
     DRP_ENTRY(drp_texture_fwd),
     DRP_ENTRY(drp_texture_bwd),

@@ -2,8 +2,9 @@
 
 ``l1_loss(pred, target)`` equals ``(pred - target).abs().mean()`` (gradient
 sign(pred - target) / n, zero at exact ties, as torch's abs) but reads both
-images once and writes the gradient in the same pass
-(``drp_l1_loss_fwd``), instead of the separate subtract / abs / mean /
+images once and keeps the gradient's signs from the same pass
+(``drp_l1_loss_sign_fwd``; the gradient itself, ``drp_l1_loss_fwd``, for
+tensors that do not start on 16 bytes), instead of the separate subtract / abs / mean /
 sign / multiply passes of the unfused expression.
 """
 import torch
@@ -19,20 +20,40 @@ class _L1(torch.autograd.Function):
         n = pred.numel()
         p = pred.contiguous()
         t = target.contiguous()
-        grad = torch.empty_like(p)
+        scale = 1.0 / n
         loss = torch.empty((), dtype=torch.float32, device=p.device)
         ws = torch.empty(_ffi.size_out("drp_l1_loss_workspace_size", n), dtype=torch.uint8, device=p.device)
-        _ffi.call("drp_l1_loss_fwd", ws.data_ptr(), ws.numel(), p.data_ptr(), t.data_ptr(), n, 1.0 / n,
-                  loss.data_ptr(), grad.data_ptr(), _ffi.stream_of(p.device))
-        ctx.save_for_backward(grad)
-        ctx.target_grad = target.requires_grad
+        if (p.data_ptr() | t.data_ptr()) & 15:
+            kept = torch.empty_like(p)
+            entry = "drp_l1_loss_fwd"
+        else:
+            kept = torch.empty((n + 3) // 4, dtype=torch.uint8, device=p.device)
+            entry = "drp_l1_loss_sign_fwd"
+        _ffi.call(entry, ws.data_ptr(), ws.numel(), p.data_ptr(), t.data_ptr(), n, scale, loss.data_ptr(),
+                  kept.data_ptr(), _ffi.stream_of(p.device))
+        ctx.save_for_backward(kept)
+        ctx.meta = (pred.shape, scale, target.requires_grad)
         return loss
 
     @staticmethod
     def backward(ctx, g):
-        grad, = ctx.saved_tensors
-        gp = grad * g
-        return gp, (-gp if ctx.target_grad else None)
+        kept, = ctx.saved_tensors
+        shape, scale, target_grad = ctx.meta
+        if kept.dtype != torch.uint8:
+            gp = kept * g
+        elif torch.is_grad_enabled() or not torch._C._has_storage(g):
+            # the gradient as a tensor of its own: autograd and vmap see the product
+            gp = _signed(kept, shape, scale, torch.ones_like(kept[:1], dtype=torch.float32)) * g
+        else:
+            gp = _signed(kept, shape, scale, g)
+        return gp, (-gp if target_grad else None)
+
+
+def _signed(signs, shape, scale, upstream):
+    grad = torch.empty(shape, dtype=torch.float32, device=signs.device)
+    _ffi.call("drp_l1_loss_bwd", signs.data_ptr(), grad.numel(), scale, upstream.data_ptr(), grad.data_ptr(),
+              _ffi.stream_of(signs.device))
+    return grad
 
 
 def l1_loss(pred, target):

@@ -264,6 +264,17 @@ int drp_l1_loss_workspace_size(long long n, size_t* bytes);
 int drp_l1_loss_fwd(void* workspace, size_t workspace_bytes, const float* pred, const float* target, long long n,
                     float scale, float* loss, float* grad, void* stream);
 
+/*
+ * drp_l1_loss_fwd that keeps the signs instead of writing the gradient, for
+ * 16-byte aligned pred and target: signs holds (n + 3) / 4 bytes, bit k (4 + k)
+ * of byte i set where element 4 i + k lies above (below) its target.  The loss
+ * equals drp_l1_loss_fwd's.  drp_l1_loss_bwd then writes grad = sign * scale *
+ * upstream[0] (one device float; grad 16-byte aligned).
+ */
+int drp_l1_loss_sign_fwd(void* workspace, size_t workspace_bytes, const float* pred, const float* target, long long n,
+                         float scale, float* loss, void* signs, void* stream);
+int drp_l1_loss_bwd(const void* signs, long long n, float scale, const float* upstream, float* grad, void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* Clip-space transform                                                     */
 /* ------------------------------------------------------------------------ */
