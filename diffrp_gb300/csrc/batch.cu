@@ -234,9 +234,8 @@ __device__ __forceinline__ int find_item_by_tile(const drp_batch_item* items, in
     return lo;
 }
 
-template <int TILE_LOG2, int TPT, bool FIT>
-__global__ void __launch_bounds__((1 << (2 * TILE_LOG2)) < 256 ? (1 << (2 * TILE_LOG2)) : 256,
-                                  TILE_LOG2 == 3 ? 12 : 4)
+template <int TILE_LOG2, int TPT, bool FIT, int NT>
+__global__ void __launch_bounds__(NT, fine_ctas<TILE_LOG2, NT>())
 batch_fine_kernel(BatchArgs a) {
     // The tile's parameters live in shared memory, filled by thread 0 with
     // the job: held in registers through the fine raster they pushed its
@@ -297,7 +296,7 @@ batch_fine_kernel(BatchArgs a) {
         }
         __syncthreads();
         if (job >= a.total_tiles) break;
-        fine_tile<TILE_LOG2, TPT, false>(ft, e);
+        fine_tile<TILE_LOG2, TPT, false, NT>(ft, e);
     }
 }
 
@@ -1703,15 +1702,14 @@ __global__ void __launch_bounds__(256) batch_clear_kernel(uint32_t* stats, unsig
     }
 }
 
-template <int TL, int TPT, bool FIT>
+template <int TL, int TPT, bool FIT, int NT = fine_threads<TL>()>
 static void launch_batch_fine(const BatchArgs& a, cudaStream_t s) {
-    constexpr int NT = (1 << (2 * TL)) < 256 ? (1 << (2 * TL)) : 256;
     // persistent grid: every resident CTA slot of the device (occupancy per
     // kernel instantiation is device-independent for one architecture)
     static std::atomic<int> per_sm{0};
     int per = per_sm.load(std::memory_order_relaxed);
     if (per == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_fine_kernel<TL, TPT, FIT>, NT, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_fine_kernel<TL, TPT, FIT, NT>, NT, 0);
         per = per > 0 ? per : 1;
         per_sm.store(per, std::memory_order_relaxed);
     }
@@ -1727,14 +1725,17 @@ static void launch_batch_fine(const BatchArgs& a, cudaStream_t s) {
         launch_tile_order(a.tile_count, a.total_tiles, a.tile_cursor, s);
         b.tile_order = a.tile_cursor;
     }
-    launch_pdl(batch_fine_kernel<TL, TPT, FIT>, dim3((unsigned)g), dim3(NT), s, b);
+    launch_pdl(batch_fine_kernel<TL, TPT, FIT, NT>, dim3((unsigned)g), dim3(NT), s, b);
     drp_note_launch();
 }
 
 template <int TL, bool FIT>
 static void launch_batch_fine(const BatchArgs& a, cudaStream_t s) {
     switch (a.tpt) {
-    case 0: launch_batch_fine<TL, 0, FIT>(a, s); break;
+    case 0:
+        if (fine_many(TL, a.total_tiles)) launch_batch_fine<TL, 0, FIT, fine_threads_many<TL>()>(a, s);
+        else launch_batch_fine<TL, 0, FIT>(a, s);
+        break;
     case 1: launch_batch_fine<TL, 1, FIT>(a, s); break;
     case 2: launch_batch_fine<TL, 2, FIT>(a, s); break;
     case 4: launch_batch_fine<TL, 4, FIT>(a, s); break;

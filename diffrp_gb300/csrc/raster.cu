@@ -123,9 +123,8 @@ struct RastEmit {
 
 // PEEL: a previous layer's keys are given (depth peeling).  Only the
 // pixel-parallel shape (TPT = 0) has a separate instantiation without them.
-template <int TILE_LOG2, int TPT, bool PEEL>
-__global__ void __launch_bounds__((1 << (2 * TILE_LOG2)) < 256 ? (1 << (2 * TILE_LOG2)) : 256,
-                                  TILE_LOG2 == 3 ? 12 : 4)
+template <int TILE_LOG2, int TPT, bool PEEL, int NT = fine_threads<TILE_LOG2>()>
+__global__ void __launch_bounds__(NT, fine_ctas<TILE_LOG2, NT>())
 fine_raster_kernel(RasterArgs a) {
     const long long tiles = (long long)a.tiles_x * a.tiles_y;
     long long tidx = (long long)blockIdx.y * tiles + blockIdx.x;  // blocks start in this order
@@ -163,7 +162,7 @@ fine_raster_kernel(RasterArgs a) {
     e.rast = reinterpret_cast<float4*>(a.rast) + b * npix;
     e.db = a.rast_db ? reinterpret_cast<float4*>(a.rast_db) + b * npix : nullptr;
     e.key = a.out_key ? a.out_key + b * npix : nullptr;
-    fine_tile<TILE_LOG2, TPT, PEEL>(ft, e);
+    fine_tile<TILE_LOG2, TPT, PEEL, NT>(ft, e);
 }
 
 // ---------------------------------------------------------------------------
@@ -227,7 +226,7 @@ constexpr long long kOrderTilesPerCTA = 8;
 
 template <int TL>
 static void launch_fine(const RasterArgs& args, int tpt, cudaStream_t s) {
-    constexpr int NT = (1 << (2 * TL)) < 256 ? (1 << (2 * TL)) : 256;
+    constexpr int NT = fine_threads<TL>(), NM = fine_threads_many<TL>();
     dim3 grid((unsigned)(args.tiles_x * args.tiles_y), (unsigned)args.B);
     // resident CTAs per SM of the instantiations (launch bounds: 4 above
     // 8-pixel tiles); the fill cursors are spent by now and hold the order
@@ -241,8 +240,13 @@ static void launch_fine(const RasterArgs& args, int tpt, cudaStream_t s) {
     }
     switch (tpt) {
     case 0:
-        if (a.prev_key) fine_raster_kernel<TL, 0, true><<<grid, NT, 0, s>>>(a);
-        else fine_raster_kernel<TL, 0, false><<<grid, NT, 0, s>>>(a);
+        if (fine_many(TL, ntiles)) {
+            if (a.prev_key) fine_raster_kernel<TL, 0, true, NM><<<grid, NM, 0, s>>>(a);
+            else fine_raster_kernel<TL, 0, false, NM><<<grid, NM, 0, s>>>(a);
+        } else {
+            if (a.prev_key) fine_raster_kernel<TL, 0, true><<<grid, NT, 0, s>>>(a);
+            else fine_raster_kernel<TL, 0, false><<<grid, NT, 0, s>>>(a);
+        }
         drp_note_launch();
         break;
     case 1: fine_raster_kernel<TL, 1, true><<<grid, NT, 0, s>>>(a); drp_note_launch(); break;

@@ -362,9 +362,9 @@ template <int TILE_LOG2, int NTHREADS>
 __device__ __forceinline__ int tile_block(int tid, int q) {
     constexpr int T = 1 << TILE_LOG2;
     constexpr int PPT = T * T / NTHREADS;
-    static_assert(PPT == 1 || (PPT == 4 && T == 32), "tile_pixel: unsupported tile shape");
+    static_assert(T * T % NTHREADS == 0 && NTHREADS >= 2 * T, "tile_pixel: unsupported tile shape");
     const int w = tid >> 5;
-    if (PPT == 4) return ((((w >> 1) << 1) | (q >> 1)) * (T / 8)) + (((w & 1) << 1) | (q & 1));
+    if (PPT == 4 && T == 32) return ((((w >> 1) << 1) | (q >> 1)) * (T / 8)) + (((w & 1) << 1) | (q & 1));
     return w + q * (NTHREADS >> 5);
 }
 
@@ -464,6 +464,27 @@ struct FineTile {
     uint32_t* stats;            // device error bits or null
 };
 
+// Threads of a fine-raster CTA: 256 (64 for 8-pixel tiles, one pixel each).
+// Pixel-parallel launches of many tiles take 128: eight CTAs per SM instead of
+// four, so that three warps wait while one prepares a tile's primitives, not
+// seven.  A tile with a long list then takes twice as long, and a launch of few
+// tiles waits for it: 16-pixel tiles, 2,080 tiles of dense meshes 158 us with
+// 256 against 266 with 128, 4,096 of 980k triangles 282 against 329; but 7,800
+// tiles 285 against 214, 23,000 (ten meshes) 445 against 405, six views of
+// 800 x 1000 (18,900) 173 against 121.  32-pixel tiles have four times the list:
+// 3,375 tiles 224 against 235, 7,300 655 against 679, 16,384 (64 views of
+// 512 x 512) 300 against 244.
+template <int TILE_LOG2>
+__host__ __device__ constexpr int fine_threads() { return TILE_LOG2 == 3 ? 64 : 256; }
+template <int TILE_LOG2>
+__host__ __device__ constexpr int fine_threads_many() { return TILE_LOG2 == 3 ? 64 : 128; }
+template <int TILE_LOG2, int NT>
+__host__ __device__ constexpr int fine_ctas() { return TILE_LOG2 == 3 ? 12 : 1024 / NT; }
+constexpr long long kFineManyTiles16 = 4864, kFineManyTiles32 = 12288;
+static inline bool fine_many(int tile_log2, long long tiles) {
+    return tile_log2 >= 4 && tiles >= (tile_log2 == 4 ? kFineManyTiles16 : kFineManyTiles32);
+}
+
 // Fine raster of one tile by one CTA, then emit(px, py, key, ndc x, ndc y)
 // for every pixel of the tile inside the viewport.
 //   TPT == 0: pixel-parallel.  The tile's 8x4 pixel blocks are handed to the
@@ -481,11 +502,10 @@ struct FineTile {
 //   TPT  > 0: groups of TPT threads walk one primitive's bbox within the tile
 //             and resolve keys with shared-memory atomicMin.
 //   PEEL = false: ft.prev is ignored (no previous layer).
-template <int TILE_LOG2, int TPT, bool PEEL, class Emit>
+template <int TILE_LOG2, int TPT, bool PEEL, int NTHREADS, class Emit>
 __device__ __forceinline__ void fine_tile(const FineTile& ft, Emit& emit) {
     constexpr int T = 1 << TILE_LOG2;
     constexpr int NPIX = T * T;
-    constexpr int NTHREADS = NPIX < 256 ? NPIX : 256;
     constexpr int PPT = NPIX / NTHREADS;
     constexpr int NBLK = NPIX / 32;  // 8x4 blocks
     constexpr int CHUNK = NTHREADS;  // primitives prepared per pass: one per thread
