@@ -412,6 +412,21 @@ __device__ __forceinline__ void atomic_add4(float4* dst, const float4& v) {
 #endif
 }
 
+// Four floats: one vector (VEC) or the n below four, the others zero.
+template <bool VEC>
+__device__ __forceinline__ void load4(const float* p, int n, float* x) {
+    if (VEC) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+        x[0] = q.x;
+        x[1] = q.y;
+        x[2] = q.z;
+        x[3] = q.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = k < n ? __ldg(p + k) : 0.f;
+    }
+}
+
 // Asynchronous copy of N bytes (4 or 16, both ends aligned to N) into shared
 // memory; a thread's copies since its last commit form a group, and wait<K>
 // returns when all but its last K groups have arrived (visible to that thread).

@@ -21,6 +21,7 @@
 //      instead, so the result never depends on the capacity.
 #include "drp_internal.h"
 #include "raster_core.cuh"
+#include "walk.cuh"
 
 namespace drp {
 
@@ -217,6 +218,104 @@ __global__ void __launch_bounds__(256) raster_bwd_kernel(RasterBwdArgs a) {
     }
 }
 
+// Backward of larger launches without gradients of rast_db, by columns
+// (walk.cuh): the pixel's triangle and its clip vertices are looked up where the
+// column enters it, and the gradients come by asynchronous copies two rows ahead.
+// What bounds it: the latency of a strip's rows.  4.8M pixels: 69 instead of 91
+// us.
+constexpr int kRasterStages = 3, kRasterRows = 8;
+struct RasterWalkShared {
+    WalkRows<3> rows;
+    float id[kRasterStages][32];
+    float4 g[kRasterStages][32];
+};
+
+__global__ void __launch_bounds__(32 * kWalkWarps, 16 / kWalkWarps) raster_bwd_walk_kernel(RasterBwdArgs a) {
+    __shared__ RasterWalkShared shared[kWalkWarps];
+    WalkStrip s;
+    if (!walk_strip(a.B, a.H, a.W, kRasterRows, s)) return;
+    RasterWalkShared& sh = shared[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, x = s.x0 + lane, W = a.W;
+    const bool in = x < W;
+    const long long view = (long long)s.b * a.H * W;
+    const float* R = a.rast + 4 * view;
+    const float4* G = reinterpret_cast<const float4*>(a.grad_rast) + view;
+    const float4* P = reinterpret_cast<const float4*>(a.pos + (long long)s.b * a.pos_view_stride);
+    float4* GP = reinterpret_cast<float4*>(a.grad_pos + (long long)s.b * a.pos_view_stride);
+    float4 p0, p1, p2, acc[3];
+    p0 = p1 = p2 = acc[0] = acc[1] = acc[2] = make_float4(0.f, 0.f, 0.f, 0.f);
+    int cur = -1, j0 = 0, j1 = 0, j2 = 0, n = 0;
+    const auto leave = [&](float* row) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) reinterpret_cast<float4*>(row)[k] = acc[k];
+        *reinterpret_cast<int4*>(row + 12) = make_int4(j0, j1, j2, 0);
+    };
+    const auto add = [&](const float* row, int quad, const float4& v) {
+        atomic_add4(GP + __float_as_int(row[12 + quad]), v);
+    };
+    const auto request = [&](int y) {
+        if (in && y < s.y1) {
+            const int st = (y - s.y0) % kRasterStages;
+            const long long p = (long long)y * W + x;
+            cp_async<4>(&sh.id[st][lane], R + 4 * p + 3);
+            cp_async<16>(&sh.g[st][lane], G + p);
+        }
+        cp_async_commit();
+    };
+    request(s.y0);
+    request(s.y0 + 1);
+    cp_async_wait<1>();  // row y0 (this lane's part, as below)
+    int i0 = 0, i1 = 0, i2 = 0;
+    int t = in ? checked_tri(sh.id[0][lane], a.tri, a.num_triangles, a.num_vertices, i0, i1, i2) : -1;
+    int st = 0;
+    const float X = pixel_ndc(x, W);
+#pragma unroll 1
+    for (int y = s.y0; y < s.y1; ++y) {
+        request(y + 2);
+        cp_async_wait<1>();  // row y + 1
+        const int stn = st + 1 == kRasterStages ? 0 : st + 1;
+        int n0 = i0, n1 = i1, n2 = i2, tn = -1;
+        if (in && y + 1 < s.y1) {
+            const float id = sh.id[stn][lane];
+            tn = t;
+            if (id != sh.id[st][lane]) tn = checked_tri(id, a.tri, a.num_triangles, a.num_vertices, n0, n1, n2);
+        }
+        const bool live = t >= 0, enter = live && t != cur;
+        walk_leave<3>(sh.rows, n, enter && cur >= 0, leave, add);
+        if (enter) {
+            cur = t;
+            j0 = i0;
+            j1 = i1;
+            j2 = i2;
+            p0 = P[i0];
+            p1 = P[i1];
+            p2 = P[i2];
+            acc[0] = acc[1] = acc[2] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (live) {
+            Shade S;
+            shade_eval_xy(p0, p1, p2, X, pixel_ndc(y, a.H), W, a.H, S);
+            const float4 g = sh.g[st][lane];
+            float4 out[3];
+            shade_grad(p0, p1, p2, S, g.x, g.y, g.z, nullptr, out);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                acc[k].x += out[k].x;
+                acc[k].y += out[k].y;
+                acc[k].z += out[k].z;
+                acc[k].w += out[k].w;
+            }
+        }
+        t = tn;
+        i0 = n0;
+        i1 = n1;
+        i2 = n2;
+        st = stn;
+    }
+    walk_leave<3>(sh.rows, n, cur >= 0, leave, add);
+    if (n) walk_drain<3>(sh.rows, n, add);
+}
+
 // ---------------------------------------------------------------------------
 // Host-side launchers.
 // ---------------------------------------------------------------------------
@@ -296,10 +395,19 @@ int launch_rasterize(const RasterArgs& a, cudaStream_t s) {
     return 0;
 }
 
+// Pixels from which the backward goes by columns: one 1024 x 1024 view takes
+// 20.7 us by pixels and 22.2 by columns, four 86.4 and 67.3.  With gradients of
+// rast_db (more arithmetic per pixel, less to gain) it stays by pixels:
+// 1400 x 1400, 82k triangles, 44.0 against 45.8 us.
+constexpr long long kWalkPixels = 1ll << 22;
+
 int launch_raster_bwd(const RasterBwdArgs& a, cudaStream_t s) {
     const long long n = (long long)a.B * a.H * a.W;
     if (n == 0) return 0;
-    raster_bwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a);
+    if (n < kWalkPixels || a.grad_db)
+        raster_bwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a);
+    else
+        raster_bwd_walk_kernel<<<walk_blocks(a.B, a.H, a.W, kRasterRows), 32 * kWalkWarps, 0, s>>>(a);
     drp_note_launch();
     return 0;
 }
