@@ -192,8 +192,14 @@ __device__ __forceinline__ float tex_coord(float u, int size) {
 struct Bilin {
     int i00, i10, i01, i11;
     float fx, fy;
-    int ix, iy;  // the tap's first texel before the boundary rule
+    int kx, ky;  // the tap's texel columns / rows as one number each (pair_key)
 };
+
+// A pair of texel indices (-1: outside) that a boundary rule gives, as one
+// number: within one rule and size equal numbers mean equal pairs.
+__device__ __forceinline__ int pair_key(int a, int b) {
+    return ((a + 1) << 2) | (b == a ? 0 : (b == a + 1 ? 1 : (b == a - 1 ? 2 : 3)));
+}
 
 __device__ __forceinline__ Bilin bilin_setup(float u, float v, int w, int h, int boundary) {
     Bilin B;
@@ -202,11 +208,11 @@ __device__ __forceinline__ Bilin bilin_setup(float u, float v, int w, int h, int
     B.fx = x - x0;
     B.fy = y - y0;
     const int ix = (int)x0, iy = (int)y0;
-    B.ix = ix;
-    B.iy = iy;
     int xa, xb, ya, yb;
     tap_pair(ix, w, boundary, xa, xb);
     tap_pair(iy, h, boundary, ya, yb);
+    B.kx = pair_key(xa, xb);
+    B.ky = pair_key(ya, yb);
     B.i00 = xa < 0 || ya < 0 ? -1 : ya * w + xa;
     B.i10 = xb < 0 || ya < 0 ? -1 : ya * w + xb;
     B.i01 = xa < 0 || yb < 0 ? -1 : yb * w + xa;
@@ -434,34 +440,82 @@ __device__ __forceinline__ float* grad_level(const TexArgs& a, int k, int n) {
     return const_cast<float*>(tex_level(a, a.grad_tex, a.grad_pyr, k, n));
 }
 
-__device__ __forceinline__ void bilin_bwd(const float* lvl, float* glvl, const Bilin& B, int w, int h, int C,
-                                          const float* g, float wl, float& gu, float& gv) {
+// The lanes (of active) whose taps are the same four texels of the same level
+// and texture, whichever repetition of the texture, or side of its border, they
+// lie in.
+__device__ __forceinline__ unsigned tap_peers(const Bilin& B, int level, int tn, bool per_view, unsigned active) {
+    // texel indices below 2^25: 28 bits each
+    const unsigned long long key = ((unsigned long long)level << 56) |
+                                   ((unsigned long long)(B.kx & 0xfffffff) << 28) |
+                                   (unsigned long long)(B.ky & 0xfffffff);
+    unsigned peers = __match_any_sync(active, key);
+    if (per_view) peers &= __match_any_sync(active, (unsigned)tn);
+    return peers;
+}
+
+// NC channels of one bilinear tap: texel gradients (one group sum of all taps'
+// values over the lanes that share the texels, NC scalar atomics per texel from
+// the lowest lane), the slopes in x and y, and the sampled values s.  lvl, glvl:
+// at the first of the channels.  What bounds it: the atomics, and the group sums
+// of warps on few texels.  A match and a sum per channel and texel instead took
+// 119 us on two 500 x 700 views of a 750 x 1000 RGB texture (now 54) and 1364 on
+// four 1400 x 1400 views of a 1024 x 1024 one, bilinear (now 516).
+template <int NC>
+__device__ __forceinline__ void bilin_bwd(const float* lvl, float* glvl, const Bilin& B, int C, const float (&g)[NC],
+                                          float wl, unsigned peers, unsigned active, float& dx, float& dy,
+                                          float (&s)[NC]) {
     const float fx = B.fx, fy = B.fy;
     const float wt[4] = {(1.f - fx) * (1.f - fy), fx * (1.f - fy), (1.f - fx) * fy, fx * fy};
     const int idx[4] = {B.i00, B.i10, B.i01, B.i11};
-    const unsigned active = __activemask();
-    float dx = 0.f, dy = 0.f;
-    for (int c = 0; c < C; ++c) {
+    float val[4 * NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
         const float gc = g[c] * wl;
         const float t00 = fetch(lvl, B.i00, C, c), t10 = fetch(lvl, B.i10, C, c);
         const float t01 = fetch(lvl, B.i01, C, c), t11 = fetch(lvl, B.i11, C, c);
+        s[c] = bilerp(B, t00, t10, t01, t11);
         dx = fmaf(gc, fmaf(1.f - fy, t10 - t00, fy * (t11 - t01)), dx);
         dy = fmaf(gc, fmaf(fx, t11 - t01, t01) - fmaf(fx, t10 - t00, t00), dy);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            float val[1] = {gc * wt[t]};
-            warp_add<1>(idx[t] >= 0 ? glvl + (long long)idx[t] * C + c : nullptr, val, active);
-        }
+        for (int t = 0; t < 4; ++t) val[NC * t + c] = gc * wt[t];
     }
-    gu = fmaf(dx, (float)w, gu);
-    gv = fmaf(dy, (float)h, gv);
+    group_sum<4 * NC>(val, peers, active);
+    if ((threadIdx.x & 31) != __ffs(peers) - 1) return;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        if (idx[t] < 0) continue;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) atomicAdd(glvl + (long long)idx[t] * C + c, val[NC * t + c]);
+    }
+}
+
+// A pixel's two levels for the channels a bilin_bwd<NC> takes, from c0 on.
+struct TexTaps {
+    Bilin B0, B1;
+    const float *P0, *P1;
+    float *G0, *G1;
+    float f;
+    unsigned peers0, peers1, active0, active1;  // active1: the lanes with f > 0
+    float dx0, dy0, dx1, dy1, dl;
+};
+
+template <int NC>
+__device__ __forceinline__ void tex_bwd_channels(TexTaps& T, int C, int c0, const float* go) {
+    float g[NC], s0[NC], s1[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) g[c] = go[c0 + c];
+    bilin_bwd<NC>(T.P0 + c0, T.G0 + c0, T.B0, C, g, T.f > 0.f ? 1.f - T.f : 1.f, T.peers0, T.active0, T.dx0, T.dy0, s0);
+    if (T.f > 0.f) {
+        bilin_bwd<NC>(T.P1 + c0, T.G1 + c0, T.B1, C, g, T.f, T.peers1, T.active1, T.dx1, T.dy1, s1);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) T.dl = fmaf(g[c], s1[c] - s0[c], T.dl);
+    }
 }
 
 // bilin_bwd of four channels from one float4 load per texel (the same
-// arithmetic per channel); q: the texels.  Lanes whose taps start at the same
-// texel (ix, iy) of the same level and texture share all four texels: one
-// match finds them, one group sum adds their 4 x 4 values and the group's
-// lowest lane issues the four float4 atomics.
+// arithmetic per channel), with float4 atomics; q: the texels.  1024 x 1024 RGBA,
+// trilinear: 64 us; with the other channel counts' code in one kernel (spills),
+// and lanes grouped by their coordinates instead of their texels, 80.
 __device__ __forceinline__ void bilin_bwd4(const Quad& q, float* glvl, const Bilin& B, int level, int tn,
                                            bool per_view, int w, int h, float4 g4, float wl, float& gu,
                                            float& gv) {
@@ -469,6 +523,7 @@ __device__ __forceinline__ void bilin_bwd4(const Quad& q, float* glvl, const Bil
     const float wt[4] = {(1.f - fx) * (1.f - fy), fx * (1.f - fy), (1.f - fx) * fy, fx * fy};
     const int idx[4] = {B.i00, B.i10, B.i01, B.i11};
     const unsigned active = __activemask();
+    const unsigned peers = tap_peers(B, level, tn, per_view, active);
     const float gc[4] = {g4.x * wl, g4.y * wl, g4.z * wl, g4.w * wl};
     const float a00[4] = {q.t00.x, q.t00.y, q.t00.z, q.t00.w}, a10[4] = {q.t10.x, q.t10.y, q.t10.z, q.t10.w};
     const float a01[4] = {q.t01.x, q.t01.y, q.t01.z, q.t01.w}, a11[4] = {q.t11.x, q.t11.y, q.t11.z, q.t11.w};
@@ -479,12 +534,6 @@ __device__ __forceinline__ void bilin_bwd4(const Quad& q, float* glvl, const Bil
         dx = fmaf(gc[c], fmaf(1.f - fy, t10 - t00, fy * (t11 - t01)), dx);
         dy = fmaf(gc[c], fmaf(fx, t11 - t01, t01) - fmaf(fx, t10 - t00, t00), dy);
     }
-    // ix, iy within +-2^24 + 1 (tex_coord's clamp): 26 bits each after the offset
-    const unsigned long long key = ((unsigned long long)level << 56) |
-                                   ((unsigned long long)((B.ix + (1 << 25)) & 0x3ffffff) << 26) |
-                                   (unsigned long long)((B.iy + (1 << 25)) & 0x3ffffff);
-    unsigned peers = __match_any_sync(active, key);
-    if (per_view) peers &= __match_any_sync(active, (unsigned)tn);
     float val[16];
 #pragma unroll
     for (int t = 0; t < 4; ++t)
@@ -504,6 +553,7 @@ __device__ __forceinline__ void bilin_bwd4(const Quad& q, float* glvl, const Bil
 
 // One pixel's gradients: texel gradients added into the levels, the uv and
 // uv_da gradients written.
+template <bool VEC4>
 __device__ __forceinline__ void tex_bwd_pixel(const TexArgs& a, long long p, const TexIn& in) {
     const float u = in.u, v = in.v;
     const int n = (int)(p / a.view_pix), tn = a.Nt == 1 ? 0 : n;
@@ -526,7 +576,7 @@ __device__ __forceinline__ void tex_bwd_pixel(const TexArgs& a, long long p, con
         const float f = L.f;
         const bool want_dl = (a.grad_uv_da || a.grad_bias) && L.interior;
         float dl = 0.f;  // d out / d lambda . grad_out
-        if (a.vec4) {
+        if constexpr (VEC4) {
             const float4 g4 = reinterpret_cast<const float4*>(a.grad_out)[p];
             const Quad q0 = fetch_quad(P0, B0);
             bilin_bwd4(q0, grad_level(a, L.l0, tn), B0, L.l0, tn, a.Nt > 1, a.lw[L.l0], a.lh[L.l0], g4,
@@ -545,16 +595,37 @@ __device__ __forceinline__ void tex_bwd_pixel(const TexArgs& a, long long p, con
                 }
             }
         } else {
-            bilin_bwd(P0, grad_level(a, L.l0, tn), B0, a.lw[L.l0], a.lh[L.l0], C, g, f > 0.f ? 1.f - f : 1.f, gu,
-                      gv);
+            // one match per level, the channels four at a time
+            TexTaps T;
+            T.f = f;
+            T.B0 = B0;
+            T.P0 = P0;
+            T.G0 = grad_level(a, L.l0, tn);
+            T.active0 = __activemask();
+            T.peers0 = tap_peers(B0, L.l0, tn, a.Nt > 1, T.active0);
+            T.active1 = __ballot_sync(T.active0, f > 0.f);
+            T.dx0 = T.dy0 = T.dx1 = T.dy1 = T.dl = 0.f;
             if (f > 0.f) {
-                const Bilin B1 = bilin_setup(u, v, a.lw[L.l1], a.lh[L.l1], a.boundary);
-                const float* P1 = tex_level(a, a.tex, a.pyr, L.l1, tn);
-                bilin_bwd(P1, grad_level(a, L.l1, tn), B1, a.lw[L.l1], a.lh[L.l1], C, g, f, gu, gv);
-                if (want_dl)
-                    for (int c = 0; c < C; ++c)
-                        dl = fmaf(g[c], bilin_value(P1, B1, C, c) - bilin_value(P0, B0, C, c), dl);
+                T.B1 = bilin_setup(u, v, a.lw[L.l1], a.lh[L.l1], a.boundary);
+                T.P1 = tex_level(a, a.tex, a.pyr, L.l1, tn);
+                T.G1 = grad_level(a, L.l1, tn);
+                T.peers1 = tap_peers(T.B1, L.l1, tn, a.Nt > 1, T.active1);
             }
+            int c0 = 0;
+            for (; c0 + 4 <= C; c0 += 4) tex_bwd_channels<4>(T, C, c0, g);
+            switch (C - c0) {
+            case 1: tex_bwd_channels<1>(T, C, c0, g); break;
+            case 2: tex_bwd_channels<2>(T, C, c0, g); break;
+            case 3: tex_bwd_channels<3>(T, C, c0, g); break;
+            default: break;
+            }
+            gu = fmaf(T.dx0, (float)a.lw[L.l0], gu);
+            gv = fmaf(T.dy0, (float)a.lh[L.l0], gv);
+            if (f > 0.f) {
+                gu = fmaf(T.dx1, (float)a.lw[L.l1], gu);
+                gv = fmaf(T.dy1, (float)a.lh[L.l1], gv);
+            }
+            if (want_dl) dl = T.dl;
         }
         if (f > 0.f && want_dl) gb = dl;
         if (f > 0.f && want_dl && a.grad_uv_da && L.da_active) {
@@ -576,6 +647,7 @@ __device__ __forceinline__ void tex_bwd_pixel(const TexArgs& a, long long p, con
 
 // kTexPix pixels per thread, blockDim.x apart (the warp's lanes take each
 // pixel together: its atomics are aggregated over the warp).
+template <bool VEC4>
 __global__ void __launch_bounds__(256, 3) tex_bwd_kernel(TexArgs a) {
     const long long base = (long long)blockIdx.x * (kTexPix * blockDim.x) + threadIdx.x;
     TexIn in[kTexPix];
@@ -584,7 +656,7 @@ __global__ void __launch_bounds__(256, 3) tex_bwd_kernel(TexArgs a) {
         if (base + j * blockDim.x < a.npix) in[j] = tex_inputs(a, base + j * blockDim.x);
 #pragma unroll
     for (int j = 0; j < kTexPix; ++j)
-        if (base + j * blockDim.x < a.npix) tex_bwd_pixel(a, base + j * blockDim.x, in[j]);
+        if (base + j * blockDim.x < a.npix) tex_bwd_pixel<VEC4>(a, base + j * blockDim.x, in[j]);
 }
 
 __device__ __forceinline__ float vadd(float a, float b) { return a + b; }
@@ -851,7 +923,9 @@ DRP_API int drp_texture_bwd(const float* tex, const float* pyr, int num_tex, int
     a.grad_bias = grad_mip_level_bias;
     if (a.npix > 0) {
         const long long per_block = 256 * drp::kTexPix;
-        drp::tex_bwd_kernel<<<(unsigned)((a.npix + per_block - 1) / per_block), 256, 0, s>>>(a);
+        const unsigned grid = (unsigned)((a.npix + per_block - 1) / per_block);
+        if (a.vec4) drp::tex_bwd_kernel<true><<<grid, 256, 0, s>>>(a);
+        else drp::tex_bwd_kernel<false><<<grid, 256, 0, s>>>(a);
         drp_note_launch();
     }
     if (levels > 1 && a.filter >= drp::kTexMipNearest) {
