@@ -502,7 +502,7 @@ constexpr int kListLanes = DRP_LIST_LANES;
 constexpr int kListBackward = 0, kListL1 = 1, kListFit = 2;
 
 template <int KIND, int LANES>
-__global__ void __launch_bounds__(256) batch_aa_bwd_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(256, KIND == kListL1 ? 0 : 3) batch_aa_bwd_kernel(BatchArgs a) {
     constexpr bool L1G = KIND != kListBackward;
     static_assert(LANES == 2 || LANES == 4, "two or four lanes per listed pixel");
     constexpr int SLOTS = 4 / LANES;  // pair slots each lane evaluates
@@ -584,15 +584,53 @@ __global__ void __launch_bounds__(256) batch_aa_bwd_kernel(BatchArgs a) {
                 const float* A = a.attr + it.attr_offset;
                 float* GA = a.grad_attr + it.attr_offset;
                 const float u = r.x, v = r.y, w = 1.0f - u - v;
-                for (int c = q; c < C; c += LANES) {
-                    const float g = aa_bwd_channel_g(at, grad, C, pix, c);
-                    const float x0 = A[(long long)i0 * C + c], x1 = A[(long long)i1 * C + c],
-                                x2 = A[(long long)i2 * C + c];
-                    atomicAdd(GA + (long long)i0 * C + c, g * u);
-                    atomicAdd(GA + (long long)i1 * C + c, g * v);
-                    atomicAdd(GA + (long long)i2 * C + c, g * w);
-                    gu = fmaf(g, x0 - x2, gu);
-                    gv = fmaf(g, x1 - x2, gv);
+                // Channels four to a lane where that leaves two lanes work (one for
+                // four channels: 154 -> 158 us on 16 dense 512 x 512 views): a
+                // quarter of the atomics.  Eight channels 109 -> 102 us (64 views),
+                // 16 channels 41 -> 37 us (one 1024 x 1024 view).  Small launches
+                // (kListL1) wait for the longest chain, not the atomics: the code's
+                // registers cost the smallest step 0.2 us.
+                if (KIND != kListL1 && (C & 3) == 0 && C >= 8 && grad.aligned() &&
+                    ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(GA)) & 15) == 0) {
+                    for (int c = 4 * q; c < C; c += 4 * LANES) {
+                        const float4 g4 = grad.load4((long long)pix * C + c);
+                        float g[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            if (at.role[k] == 0) continue;
+                            const bool own = at.role[k] == 1;
+                            const float4 n4 = own ? g4 : grad.load4((long long)at.tgt[k] * C + c);
+                            const float wk = own ? -at.wt[k] : at.wt[k];
+                            g[0] = fmaf(wk, n4.x, g[0]);
+                            g[1] = fmaf(wk, n4.y, g[1]);
+                            g[2] = fmaf(wk, n4.z, g[2]);
+                            g[3] = fmaf(wk, n4.w, g[3]);
+                        }
+                        const float4 x0 = *reinterpret_cast<const float4*>(A + (long long)i0 * C + c);
+                        const float4 x1 = *reinterpret_cast<const float4*>(A + (long long)i1 * C + c);
+                        const float4 x2 = *reinterpret_cast<const float4*>(A + (long long)i2 * C + c);
+                        atomic_add4(reinterpret_cast<float4*>(GA + (long long)i0 * C + c),
+                                    make_float4(g[0] * u, g[1] * u, g[2] * u, g[3] * u));
+                        atomic_add4(reinterpret_cast<float4*>(GA + (long long)i1 * C + c),
+                                    make_float4(g[0] * v, g[1] * v, g[2] * v, g[3] * v));
+                        atomic_add4(reinterpret_cast<float4*>(GA + (long long)i2 * C + c),
+                                    make_float4(g[0] * w, g[1] * w, g[2] * w, g[3] * w));
+                        gu = fmaf(g[3], x0.w - x2.w, fmaf(g[2], x0.z - x2.z,
+                                                     fmaf(g[1], x0.y - x2.y, fmaf(g[0], x0.x - x2.x, gu))));
+                        gv = fmaf(g[3], x1.w - x2.w, fmaf(g[2], x1.z - x2.z,
+                                                     fmaf(g[1], x1.y - x2.y, fmaf(g[0], x1.x - x2.x, gv))));
+                    }
+                } else {
+                    for (int c = q; c < C; c += LANES) {
+                        const float g = aa_bwd_channel_g(at, grad, C, pix, c);
+                        const float x0 = A[(long long)i0 * C + c], x1 = A[(long long)i1 * C + c],
+                                    x2 = A[(long long)i2 * C + c];
+                        atomicAdd(GA + (long long)i0 * C + c, g * u);
+                        atomicAdd(GA + (long long)i1 * C + c, g * v);
+                        atomicAdd(GA + (long long)i2 * C + c, g * w);
+                        gu = fmaf(g, x0 - x2, gu);
+                        gv = fmaf(g, x1 - x2, gv);
+                    }
                 }
             }
         }
@@ -840,9 +878,8 @@ __device__ __forceinline__ void store4(float* p, int n, const float (&x)[4]) {
 // One thread per pixel with segmented shuffles took 1270 warp instructions
 // per 32 pixels on 64 views of 512 x 512 x 8 channels, most of them predicated
 // shuffle steps and pair evaluation for a lane or two at a time; this takes
-// about 500, and the pass
-// 516 instead of 951 us (step 937 instead of 1414); on one 1024 x 1024 view 65
-// instead of 77 us (127 instead of 137).
+// about 500, and the pass 516 instead of 951 us; on one 1024 x 1024 view 65
+// instead of 77 us.
 // Floats per shared row: 24 attribute sums (per four channels three vertices),
 // three position sums (x, y, 0, w), the vertex indices; eight lanes' float4
 // stores cover the banks.
