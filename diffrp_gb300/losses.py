@@ -45,7 +45,7 @@ class _L1(torch.autograd.Function):
             # the gradient as a tensor of its own: autograd and vmap see the product
             gp = _signed(kept, shape, scale, torch.ones_like(kept[:1], dtype=torch.float32)) * g
         else:
-            gp = _signed(kept, shape, scale, g)
+            gp = _signed(kept, shape, scale, g.resolve_neg())
         return gp, (-gp if target_grad else None)
 
 
