@@ -846,9 +846,9 @@ def kernel_breakdown(dev, verts, f, attr, mvp, target, reps=10, tuned=None, batc
         # rast, colour and output gradient read once; vertex / attribute
         # gradients written once
         "batch_backward": P * (16 + 4 * C + 4 * C) + V * (16 + 4 * C) * 2 + F * 12,
-        # rast, colour and output written, target read; vertex / attribute
-        # gradients written (no sign-gradient image)
-        "batch_forward_l1_grad": P * (16 + 4 * C * 3) + V * (16 + 4 * C) * 2 + F * 12,
+        # rast and output written, target read; vertex / attribute gradients
+        # written (no colour image, no sign-gradient image)
+        "batch_forward_l1_grad": P * (16 + 4 * C * 2) + V * (16 + 4 * C) * 2 + F * 12,
     }
     times = {}
     for name, fn in ops.items():
