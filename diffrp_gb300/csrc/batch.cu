@@ -83,13 +83,18 @@ struct BatchArgs {
 // kSetupFill: append to the exact lists (after the scan); kSetupBins: setup,
 // record and append to fixed-depth bins in one pass.
 constexpr int kSetupCount = 0, kSetupFill = 1, kSetupBins = 2;
-// CTAs per 256-triangle block of the map, and triangles per CTA: the work is
-// a chain of dependent loads per triangle, so smaller CTAs spread one mesh's
-// few hundred map blocks over every SM.
-constexpr int kSetupSplit = 4, kSetupTris = 256 / kSetupSplit;
+// CTAs per 256-triangle block of the map: the work is a chain of dependent
+// loads per triangle, so smaller CTAs spread one mesh's few hundred map blocks
+// over every SM.  The fill's chain is short and large meshes wait for its CTAs to
+// start: two blocks of 128 triangles instead of four of 64 take 101 instead of
+// 135 us for four views of 2.09M triangles and 167 instead of 248 for 16 of 980k
+// (the count pass with two: 395 against 383, 679 against 654).
+__host__ __device__ constexpr int setup_split(int mode) { return mode == kSetupFill ? 2 : 4; }
+constexpr int kSetupSplitMost = 4;
 
 template <int TILE_LOG2, int MODE>
-__global__ void __launch_bounds__(2 * kSetupTris) batch_setup_bin_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(2 * 256 / setup_split(MODE)) batch_setup_bin_kernel(BatchArgs a) {
+    constexpr int kSetupSplit = setup_split(MODE), kSetupTris = 256 / kSetupSplit;
     pdl_wait();
     pdl_launch_dependents();
     constexpr bool FILL = MODE == kSetupFill;
@@ -1784,17 +1789,18 @@ static void launch_batch_fine(const BatchArgs& a, cudaStream_t s) {
 
 template <int TL>
 static void launch_batch_raster(const BatchArgs& a, cudaStream_t s) {
+    constexpr int kSplit = setup_split(kSetupCount), kTris = 256 / kSplit, kFillSplit = setup_split(kSetupFill);
     if (a.n_prim_blocks > 0 && a.bin_depth) {
-        launch_pdl(batch_setup_bin_kernel<TL, kSetupBins>, dim3((unsigned)(a.n_prim_blocks * kSetupSplit)),
-                   dim3(a.aa_records ? 2 * kSetupTris : kSetupTris), s, a);
+        launch_pdl(batch_setup_bin_kernel<TL, kSetupBins>, dim3((unsigned)(a.n_prim_blocks * kSplit)),
+                   dim3(a.aa_records ? 2 * kTris : kTris), s, a);
         drp_note_launch();
     } else if (a.n_prim_blocks > 0) {
-        launch_pdl(batch_setup_bin_kernel<TL, kSetupCount>, dim3((unsigned)(a.n_prim_blocks * kSetupSplit)),
-                   dim3(a.aa_records ? 2 * kSetupTris : kSetupTris), s, a);
+        launch_pdl(batch_setup_bin_kernel<TL, kSetupCount>, dim3((unsigned)(a.n_prim_blocks * kSplit)),
+                   dim3(a.aa_records ? 2 * kTris : kTris), s, a);
         drp_note_launch();
         launch_tile_scan(a.tile_count, a.tile_offset, a.tile_cursor, a.total_tiles, a.chunk_sums,
                          reinterpret_cast<unsigned long long*>(a.stats), s);
-        batch_setup_bin_kernel<TL, kSetupFill><<<(unsigned)(a.n_prim_blocks * kSetupSplit), kSetupTris, 0, s>>>(a);
+        batch_setup_bin_kernel<TL, kSetupFill><<<(unsigned)(a.n_prim_blocks * kFillSplit), 256 / kFillSplit, 0, s>>>(a);
         drp_note_launch();
     } else {
         cudaMemsetAsync(a.tile_offset, 0, sizeof(uint32_t) * a.total_tiles, s);
@@ -2044,7 +2050,7 @@ static int batch_common(void* ws, size_t ws_bytes, const drp_batch_item* items, 
     if (!ws || (reinterpret_cast<uintptr_t>(ws) & 255)) return bfail("batch: workspace must be 256-byte aligned");
     if (!items || num_items <= 0 || !pos || !tri || !attr) return bfail("batch: null table or buffer");
     if ((prim_blocks > 0 && !prim_block_map) || (pixel_blocks > 0 && !pixel_block_map) || prim_blocks < 0 ||
-        pixel_blocks < 0 || prim_blocks > 0x7fffffffll / drp::kSetupSplit || pixel_blocks > 0x7fffffffll)
+        pixel_blocks < 0 || prim_blocks > 0x7fffffffll / drp::kSetupSplitMost || pixel_blocks > 0x7fffffffll)
         return bfail("batch: bad block maps");
     if ((reinterpret_cast<uintptr_t>(pos) & 15)) return bfail("batch: pos must be 16-byte aligned");
     if (list_capacity > 0x7fffffffull) return bfail("batch: list_capacity above 2^31 - 1");
