@@ -361,7 +361,10 @@ class BatchRenderer:
             self.last_max_tile = int(words[3])
             self._capacity = max(cap, int(needed * 1.25) + 4096)
             self._depth = self._choose_depth(self.last_max_tile, needed)
-            if needed > cap:
+            # Tiles whose lists were too short were exact but slow; what the
+            # call wrote is written again from whole lists, but gradients are
+            # added to what is there: formed twice, they would count twice.
+            if needed > cap and entry != "drp_batch_fit_l1":
                 ws = self._workspace(self._capacity)
                 _ffi.call(entry, ws.data_ptr(), ws.numel(), *args, self._capacity, 0, *bufs, *tail)
         else:
