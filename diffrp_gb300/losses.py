@@ -8,6 +8,8 @@ tensors that do not start on 16 bytes), instead of the separate subtract / abs /
 sign / multiply passes of the unfused expression.
 """
 import torch
+from torch.autograd.forward_ad import unpack_dual
+from torch.utils._python_dispatch import _get_current_dispatch_mode
 
 from . import _ffi
 
@@ -41,19 +43,42 @@ class _L1(torch.autograd.Function):
         shape, scale, target_grad = ctx.meta
         if kept.dtype != torch.uint8:
             gp = kept * g
-        elif torch.is_grad_enabled() or not torch._C._has_storage(g):
-            # the gradient as a tensor of its own: autograd and vmap see the product
-            gp = _signed(kept, shape, scale, torch.ones_like(kept[:1], dtype=torch.float32)) * g
         else:
-            gp = _signed(kept, shape, scale, g.resolve_neg())
+            grad = torch.empty(shape, dtype=torch.float32, device=kept.device)
+            if not _number_in_memory(g, grad):
+                gp = _decode(kept, shape, scale) * g
+            elif torch.is_grad_enabled():  # autograd sees the product
+                gp = _signed(kept, scale, torch.ones_like(kept[:1], dtype=torch.float32), grad) * g
+            else:
+                gp = _signed(kept, scale, g.resolve_neg(), grad)
         return gp, (-gp if target_grad else None)
 
 
-def _signed(signs, shape, scale, upstream):
-    grad = torch.empty(shape, dtype=torch.float32, device=signs.device)
+def _number_in_memory(g, grad):
+    """Whether the upstream gradient is only a number that a kernel can read,
+    and grad (just allocated) only memory that it can write.  Not so: under a
+    dispatch mode (a trace) or a functorch transform, with a tangent, for a
+    batch of gradients, a subclass or a zero without memory; those take torch's
+    operators."""
+    if _get_current_dispatch_mode() is not None or type(g) is not torch.Tensor:
+        return False
+    try:
+        return bool(g.data_ptr() and grad.data_ptr()) and unpack_dual(g).tangent is None
+    except RuntimeError:  # a wrapper around the tensor that has the memory
+        return False
+
+
+def _signed(signs, scale, upstream, grad):
     _ffi.call("drp_l1_loss_bwd", signs.data_ptr(), grad.numel(), scale, upstream.data_ptr(), grad.data_ptr(),
               _ffi.stream_of(signs.device))
     return grad
+
+
+def _decode(signs, shape, scale):
+    """drp_l1_loss_bwd's gradient for an upstream of one, by torch's operators."""
+    bits = signs.unsqueeze(1) >> torch.arange(4, dtype=torch.uint8, device=signs.device)
+    sign = (bits & 1).to(torch.float32) - ((bits >> 4) & 1).to(torch.float32)
+    return sign.reshape(-1)[:shape.numel()].reshape(shape) * scale
 
 
 def l1_loss(pred, target):
