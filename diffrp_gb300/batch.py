@@ -54,6 +54,7 @@ def _register():
         "drp_batch_block_maps": [P, I, P, P],
         "drp_batch_workspace_size": [LL, LL, ULL, ctypes.POINTER(ctypes.c_size_t)],
         "drp_batch_aa_state_size": [LL, ctypes.POINTER(ctypes.c_size_t)],
+        "drp_batch_fit_words_size": [LL, ctypes.POINTER(ctypes.c_size_t)],
         "drp_batch_forward": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL, ctypes.c_uint,
                               P, P, P, P, LL, P],
         "drp_batch_render": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL, ctypes.c_uint,
@@ -264,8 +265,11 @@ class BatchRenderer:
         return out
 
     # -- execution -------------------------------------------------------------------
-    def _workspace(self, cap):
+    def _workspace(self, cap, fit=False):
+        """fit: with the pixel words of a gradient-forming forward."""
         nbytes = _ffi.size_out("drp_batch_workspace_size", self.total_prims, self.total_tiles, cap)
+        if fit:
+            nbytes += _ffi.size_out("drp_batch_fit_words_size", self.total_pixels)
         return self._wsh.get(nbytes, self.device)
 
     def _choose_depth(self, max_tile, needed):
@@ -323,12 +327,13 @@ class BatchRenderer:
         npix = self.total_pixels
         bufs = (rast.data_ptr(), None if color is None else color.data_ptr(), optr, fptr, npix)
         self._fwd_gen += 1
-        ws = self._workspace(cap)
+        fit = l1 is not None and len(l1) == 7
+        ws = self._workspace(cap, fit)
         stream = _ffi.stream_of(self.device)
         args = (self._items_dev.data_ptr(), len(self.items), self._pmap.data_ptr(), self.prim_blocks,
                 self._xmap.data_ptr(), self.pixel_blocks, self.total_prims, self.total_tiles, pos.data_ptr(),
                 self.tri.data_ptr(), attr.data_ptr(), self.nbr.data_ptr(), self.tile_log2, self.threads_per_tri)
-        if l1 is not None and len(l1) == 7:
+        if fit:
             # the loss's gradient formed in the same pass: (target, scale,
             # block_loss, loss, grad_pos, grad_attr, buffer the call zeroes
             # first or None)
@@ -364,7 +369,7 @@ class BatchRenderer:
             # Tiles whose lists were too short were exact but slow; what the
             # call wrote is written again from whole lists, but gradients are
             # added to what is there: formed twice, they would count twice.
-            if needed > cap and entry != "drp_batch_fit_l1":
+            if needed > cap and not fit:
                 ws = self._workspace(self._capacity)
                 _ffi.call(entry, ws.data_ptr(), ws.numel(), *args, self._capacity, 0, *bufs, *tail)
         else:

@@ -438,13 +438,14 @@ struct ItemGrad<true> {
     }
 };
 
-// Launches of at least this many pixels form the loss and its gradient with
-// batch_fit_kernel, smaller ones with batch_aa_l1_grad_kernel, whose shorter
-// chain per pixel is what counts while the regions fill only part of the chip:
-// one view of 400 x 400 takes 58.5 with the first against 55.3 us per step with
-// the second at 3 channels and 68.2 against 63.8 at 8; 724 x 724 84.2 against
-// 88.6 and 81.2 against 84.0 (but 12 channels 6 percent more); from 1024 x 1024
-// on 3 to 8 and 16 channels are 7 to 40 percent faster, 12 even.
+// Launches of at least this many pixels, with room in the workspace for the
+// pixel words, form the loss and its gradient with batch_fit_kernel, others with
+// batch_aa_l1_grad_kernel, whose shorter chain per pixel is what counts while the
+// regions fill only part of the chip: one view of 400 x 400 takes 58.5 with the
+// first against 55.3 us per step with the second at 3 channels and 68.2 against
+// 63.8 at 8; 724 x 724 84.2 against 88.6 and 81.2 against 84.0 (but 12 channels 6
+// percent more); from 1024 x 1024 on 3 to 8 and 16 channels are 7 to 40 percent
+// faster, 12 even.
 constexpr long long kFitPixels = 1ll << 20;
 
 // batch_fit_kernel takes regions of 32 x 16 pixels, a fixed number per raster
@@ -1664,22 +1665,26 @@ BatchLayout batch_layout(long long total_prims, long long total_tiles, unsigned 
 }
 
 // Antialias state block: list count at 0, per-pixel flags at 256, the pixel
-// list (int32) after them, then the pixel words.
-static size_t aa_state_bytes(long long total_pixels, size_t* list_off, size_t* words_off) {
-    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-    const size_t lo = up(256 + (size_t)total_pixels);
-    const size_t wo = up(lo + (size_t)total_pixels * 4);
+// list (int32) after them.  No entry is told the block's size, so this layout
+// belongs to the ABI version: scratch that a later form wants goes elsewhere.
+static size_t aa_state_bytes(long long total_pixels, size_t* list_off) {
+    const size_t flags_end = 256 + (size_t)total_pixels;
+    const size_t lo = (flags_end + 255) / 256 * 256;
     if (list_off) *list_off = lo;
-    if (words_off) *words_off = wo;
-    return wo + (size_t)total_pixels * 4;
+    return lo + (size_t)total_pixels * 4;
+}
+
+// Pixel words of batch_fit_kernel: they follow the workspace, whose size the
+// entries are told.
+static size_t fit_words_bytes(long long total_pixels) {
+    return total_pixels >= kFitPixels ? (size_t)total_pixels * 4 : 0;
 }
 
 static void carve_aa_state(BatchArgs& a, void* state, long long total_pixels) {
     if (!state) return;
-    size_t lo = 0, wo = 0;
-    aa_state_bytes(total_pixels, &lo, &wo);
+    size_t lo = 0;
+    aa_state_bytes(total_pixels, &lo);
     char* p = static_cast<char*>(state);
-    a.aa_words = reinterpret_cast<uint32_t*>(p + wo);
     a.aa_count = reinterpret_cast<unsigned*>(p);
     a.aa_flags = reinterpret_cast<unsigned char*>(p + 256);
     a.aa_list = reinterpret_cast<int*>(p + lo);
@@ -2030,7 +2035,13 @@ DRP_API int drp_batch_block_maps(const drp_batch_item* items, int num_items, int
 
 DRP_API int drp_batch_aa_state_size(long long total_pixels, size_t* bytes) {
     if (!bytes || total_pixels <= 0) return bfail("drp_batch_aa_state_size: bad arguments");
-    *bytes = drp::aa_state_bytes(total_pixels, nullptr, nullptr);
+    *bytes = drp::aa_state_bytes(total_pixels, nullptr);
+    return DRP_STATUS_OK;
+}
+
+DRP_API int drp_batch_fit_words_size(long long total_pixels, size_t* bytes) {
+    if (!bytes || total_pixels <= 0) return bfail("drp_batch_fit_words_size: bad arguments");
+    *bytes = drp::fit_words_bytes(total_pixels);
     return DRP_STATUS_OK;
 }
 
@@ -2220,7 +2231,9 @@ static int batch_fit_l1(const char* who, bool full_color, void* workspace, size_
     a.color = color;
     a.out = out;
     carve_aa_state(a, aa_state, total_pixels);
-    a.fit = total_pixels >= drp::kFitPixels;
+    const size_t words = drp::fit_words_bytes(total_pixels);
+    a.fit = words > 0 && workspace_bytes >= L.total + words;
+    a.aa_words = a.fit ? reinterpret_cast<uint32_t*>(static_cast<char*>(workspace) + L.total) : nullptr;
     a.emit_color = full_color;  // else the loss pass stores the listed pixels' colours only
     a.emit_out = false;  // the fused antialias + loss pass writes every output pixel
     a.aa_records = true;

@@ -415,7 +415,7 @@ int drp_batch_workspace_size(long long total_prims, long long total_tiles, unsig
  * raises the u32 at byte 12 to its count.
  * aa_state (may be NULL; drp_batch_aa_state_size(total_pixels) bytes,
  * 256-byte aligned): the antialias pass records there which pixels a
- * blending pair touches (a flag per pixel and a list of them, with scratch), so that
+ * blending pair touches (a flag per pixel and a list of them), so that
  * drp_batch_backward evaluates the antialias terms of those pixels only.
  */
 int drp_batch_forward(void* workspace, size_t workspace_bytes, const drp_batch_item* items, int num_items,
@@ -443,6 +443,14 @@ int drp_batch_render(void* workspace, size_t workspace_bytes, const drp_batch_it
 /* Bytes of the antialias state block of drp_batch_forward (total_pixels =
  * totals[2] of drp_batch_plan). */
 int drp_batch_aa_state_size(long long total_pixels, size_t* bytes);
+
+/*
+ * Bytes that the large-launch form of drp_batch_fit_l1 / drp_batch_forward_l1_grad
+ * uses of the workspace after drp_batch_workspace_size bytes: 0 below 2^20
+ * pixels, where there is no such form.  With a smaller workspace those entries
+ * take the form for small launches.
+ */
+int drp_batch_fit_words_size(long long total_pixels, size_t* bytes);
 
 /*
  * drp_batch_forward with the mean-absolute-error loss against target (image
@@ -492,9 +500,10 @@ int drp_batch_forward_l1_grad(void* workspace, size_t workspace_bytes, const drp
 
 /*
  * drp_batch_forward_l1_grad without the colour image: color (image floats)
- * is scratch, of which a large launch writes only the unblended colours of
- * the pixels a blending pair touches (the other pixels' colours are
- * interpolated where they are needed and never stored).  All other arguments, outputs and
+ * is scratch, of which the large-launch form (drp_batch_fit_words_size) writes
+ * only the unblended colours of the pixels a blending pair touches (the other
+ * pixels' colours are interpolated where they are needed and never stored);
+ * the small-launch form writes all of it.  All other arguments, outputs and
  * limits are drp_batch_forward_l1_grad's.  No counterpart in the reference.
  */
 int drp_batch_fit_l1(void* workspace, size_t workspace_bytes, const drp_batch_item* items, int num_items,
