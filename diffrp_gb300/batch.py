@@ -269,8 +269,13 @@ class BatchRenderer:
         """fit: with the pixel words of a gradient-forming forward."""
         nbytes = _ffi.size_out("drp_batch_workspace_size", self.total_prims, self.total_tiles, cap)
         if fit:
-            nbytes += _ffi.size_out("drp_batch_fit_words_size", self.total_pixels)
+            nbytes += self._fit_words()
         return self._wsh.get(nbytes, self.device)
+
+    def _fit_words(self):
+        """Bytes of the pixel words: 0 where the gradient-forming forward takes
+        the form for small launches, which fills the whole colour image."""
+        return _ffi.size_out("drp_batch_fit_words_size", self.total_pixels)
 
     def _choose_depth(self, max_tile, needed):
         if self.bin_depth_mode is not None:
@@ -612,7 +617,9 @@ class _BatchL1GradFn(torch.autograd.Function):
         renderer._forward_raw(pos, attr, rast, color, out, (target, scale, block_loss, loss, gpos, gattr, gbuf),
                               flags=flags)
         ctx.gen = renderer._fwd_gen
-        ctx.save_for_backward(pos, attr, target, out, gbuf, flags, rast, color)
+        # the state holds the pixel list alone, which a backward through the
+        # images cannot use; the large launch's color is scratch
+        ctx.save_for_backward(pos, attr, target, out, gbuf, rast, None if renderer._fit_words() else color)
         return loss, out
 
     @staticmethod
@@ -643,13 +650,13 @@ class _BatchL1GradFn(torch.autograd.Function):
                 cr._backward_raw(pos[c.rows], attr, rast, color, gout[c.floats], grad_pos[c.rows], grad_attr,
                                  cr._fwd_gen, aa_flags=flags)
             return grad_pos, grad_attr, None, None
-        _, rast, color = saved[5:]
-        # the gradient-forming forward keeps no colour image (its color buffer
-        # is scratch) and fills only the state's pixel list, not its per-pixel
-        # flags: the colours are interpolated again, and the backward
-        # evaluates every pixel's antialias terms itself
-        color = torch.empty_like(color)
-        _ffi.call("drp_batch_colors", r._items_dev.data_ptr(), len(r.items), r._xmap.data_ptr(), r.pixel_blocks,
-                  r.tri.data_ptr(), attr.data_ptr(), rast.data_ptr(), color.data_ptr(), _ffi.stream_of(pos.device))
+        # without the state's per-pixel flags the backward evaluates every
+        # pixel's antialias terms itself
+        rast, color = saved[5:]
+        if color is None:
+            color = torch.empty_like(out)
+            _ffi.call("drp_batch_colors", r._items_dev.data_ptr(), len(r.items), r._xmap.data_ptr(), r.pixel_blocks,
+                      r.tri.data_ptr(), attr.data_ptr(), rast.data_ptr(), color.data_ptr(),
+                      _ffi.stream_of(pos.device))
         r._backward_raw(pos, attr, rast, color, gout, grad_pos, grad_attr, ctx.gen)
         return grad_pos, grad_attr, None, None
