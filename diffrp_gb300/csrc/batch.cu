@@ -465,21 +465,22 @@ __device__ __forceinline__ float* fit_loss_slot(const BatchArgs& a, long long i)
 }
 
 // The loss from the regions' sums: every CTA adds a contiguous slice of them
-// and leaves its sum in the slice's first slot; the CTA that arrives last (a
-// counter the forward's first kernel zeroed; nobody waits) adds the slices.
-// Fixed slices, fixed order within each: reproducible.  One CTA adding every
-// partial took 27 us of the 64-view step.
+// and leaves its sum in the slice's first slot and the sum's error in the second
+// (a slice of one has none); the CTA that arrives last (a counter the forward's
+// first kernel zeroed; nobody waits) adds the slices.  Fixed slices, fixed order
+// within each: reproducible.  One CTA adding every partial took 27 us of the
+// 64-view step.
 __device__ __forceinline__ void fit_loss(const BatchArgs& a) {
-    __shared__ float total;
     __shared__ bool last;
     const long long n = a.total_tiles * fit_regions_per_tile(a.tile_log2);
     const long long per = (n + gridDim.x - 1) / gridDim.x;
     const long long b0 = blockIdx.x * per, b1 = b0 + per < n ? b0 + per : n;
     float s = 0.f, c = 0.f;
     for (long long i = b0 + threadIdx.x; i < b1; i += blockDim.x) two_sum(s, c, *fit_loss_slot(a, i));
-    block_sum_pairs<kFinalThreads>(s, c, 1.0f, &total);
+    const float2 slice = block_sum_pairs<kFinalThreads>(s, c);
     if (threadIdx.x == 0) {
-        if (b0 < b1) *fit_loss_slot(a, b0) = total;
+        if (b0 < b1) *fit_loss_slot(a, b0) = slice.x;
+        if (b0 + 1 < b1) *fit_loss_slot(a, b0 + 1) = slice.y;
         __threadfence();
         last = atomicAdd(a.loss_count, 1u) == gridDim.x - 1;
     }
@@ -487,8 +488,12 @@ __device__ __forceinline__ void fit_loss(const BatchArgs& a) {
     if (!last) return;
     __threadfence();
     s = c = 0.f;
-    for (long long b = threadIdx.x * per; b < n; b += blockDim.x * per) two_sum(s, c, __ldcg(fit_loss_slot(a, b)));
-    block_sum_pairs<kFinalThreads>(s, c, a.l1_scale, a.loss);
+    for (long long b = threadIdx.x * per; b < n; b += blockDim.x * per) {
+        two_sum(s, c, __ldcg(fit_loss_slot(a, b)));
+        if (per > 1 && b + 1 < n) c += __ldcg(fit_loss_slot(a, b + 1));
+    }
+    const float2 sum = block_sum_pairs<kFinalThreads>(s, c);
+    if (threadIdx.x == 0) *a.loss = (sum.x + sum.y) * a.l1_scale;
 }
 
 // Lanes per listed pixel in batch_aa_bwd_kernel.  Two lanes cover twice the
@@ -994,7 +999,7 @@ __device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item
         cl.plain |= 1u << r;
         if (w[r + 1] & ~kPixSil) cl.live |= 1u << r;
     }
-    float sum = 0.f;
+    float sum = 0.f, low = 0.f;
     unsigned listed, blended;
     const auto depth = [&](int pix, int, int) { return reinterpret_cast<const float*>(R + pix)[2]; };
     if (warp_pairs<ROWS>(depth, a.aa_rec + it.prim_offset * 2, W, H, x0, y0, y1, w, side, sh, listed, blended)) {
@@ -1062,9 +1067,13 @@ __device__ __noinline__ float fit_pairs(const BatchArgs& a, const drp_batch_item
                 source();
             }
             store4<VEC>(a.out + prow, C - cg, val);
+            if (LOSS) {
+                float s4 = 0.f;
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (LOSS && (VEC || cg + c < C)) sum += fabsf(val[c] - tg[c]);
+                for (int c = 0; c < 4; ++c)
+                    if (VEC || cg + c < C) s4 += fabsf(val[c] - tg[c]);
+                kahan_add(sum, low, s4);
+            }
         }
     }
     if (C > 32) cl.live = 0u;
@@ -1102,7 +1111,7 @@ __device__ __forceinline__ float fit_walk(const BatchArgs& a, const drp_batch_it
     const float4* P = reinterpret_cast<const float4*>(a.pos) + it.pos_offset;
     const float X = fmaf((float)(2 * x + 1), __frcp_rn((float)W), -1.0f), rh = __frcp_rn((float)it.height);
     const f32x2 minus1 = pack2(-1.0f, -1.0f);
-    float s = 0.f;
+    float s = 0.f, low = 0.f;
     int n = 0;
     // the column's triangle: sums (vertex i, channels 2 k, 2 k + 1), position sums, vertices
     f32x2 acc[3][2 * NG];
@@ -1245,7 +1254,7 @@ __device__ __forceinline__ float fit_walk(const BatchArgs& a, const drp_batch_it
             if ((cl.listed & bit) && !a.emit_color)  // for the listed pixels' kernel
                 store4<VEC>(a.color + row + 4 * g, C - 4 * g, v4);
         }
-        if (cl.plain & bit) s += sr;
+        if (cl.plain & bit) kahan_add(s, low, sr);
         if (live) {
             float4 g3[3];
             uv_grad_fast(P[i0], P[i1], P[i2], X, fmaf((float)(2 * yy + 1), rh, -1.0f), gu, gv, g3);
@@ -1292,7 +1301,7 @@ __device__ __forceinline__ float fit_rows(const BatchArgs& a, const drp_batch_it
     const long long image_offset = it.image_offset;
     const float X = fmaf((float)(2 * x + 1), __frcp_rn((float)W), -1.0f), rh = __frcp_rn((float)it.height);
     const float sc = a.l1_scale;
-    float s = 0.f;
+    float s = 0.f, low = 0.f;
     int pix = y0 * W + x;
 #pragma unroll 1
     for (int yy = y0; yy < y1; ++yy, pix += W) {
@@ -1319,7 +1328,7 @@ __device__ __forceinline__ float fit_rows(const BatchArgs& a, const drp_batch_it
         float* rw = sh.rows[__popc(live_mask & ((1u << lane) - 1u))];
         if (live) *reinterpret_cast<int4*>(rw + 36) = make_int4(i0, i1, i2, 0);
         const float u = r.x, v = r.y, w = 1.0f - u - v;
-        float gu = 0.f, gv = 0.f;
+        float gu = 0.f, gv = 0.f, sr = 0.f;
 #pragma unroll 1
         for (int c0 = 0; c0 < C; c0 += 8) {
             const int ng = C - c0 > 4 ? 2 : 1;
@@ -1333,7 +1342,7 @@ __device__ __forceinline__ float fit_rows(const BatchArgs& a, const drp_batch_it
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const float d = plain && (VEC || cg + k < C) ? val[k] - tv[gi][k] : 0.f;
-                    s += fabsf(d);
+                    sr += fabsf(d);
                     g[k] = l1_sign_fast(d, sc);
                 }
                 if (plain) store4<VEC>(a.out + row + cg, C - cg, val);
@@ -1364,6 +1373,7 @@ __device__ __forceinline__ float fit_rows(const BatchArgs& a, const drp_batch_it
             else if (last) fit_drain<1, true, VEC>(a, it, sh, n, c0);
             else fit_drain<2, false, VEC>(a, it, sh, n, c0);
         }
+        kahan_add(s, low, sr);
     }
     return s;
 }

@@ -479,15 +479,22 @@ __device__ __forceinline__ void two_sum(float& s, float& c, float x) {
     c += err;
 }
 
+// Kahan's running sum s of positive terms, c its lost low part.
+__device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
+    const float y = x - c, t = s + y;
+    c = (t - s) - y;
+    s = t;
+}
+
 // Threads of the block that forms a loss from its per-block partials.
 constexpr int kFinalThreads = 256;
 
-// *out = scale * (sum of the block's (s, c) float pairs), by one whole block of
-// NT threads: a fixed shuffle tree within warps and across them.  Every thread
-// of the block calls it (it has a barrier, and one before it may be called
-// again is the caller's).
+// The sum of the block's (s, c) float pairs, as a pair that thread 0 gets, by one
+// whole block of NT threads: a fixed shuffle tree within warps and across them.
+// Every thread of the block calls it (it has a barrier, and one before it may be
+// called again is the caller's).
 template <int NT>
-__device__ __forceinline__ void block_sum_pairs(float s, float c, float scale, float* out) {
+__device__ __forceinline__ float2 block_sum_pairs(float s, float c) {
     static_assert(NT % 32 == 0 && NT <= 1024, "block_sum_pairs: whole warps, at most 1024 threads");
     __shared__ float warp_s[NT / 32], warp_c[NT / 32];
 #pragma unroll
@@ -501,17 +508,19 @@ __device__ __forceinline__ void block_sum_pairs(float s, float c, float scale, f
         warp_c[threadIdx.x >> 5] = c;
     }
     __syncthreads();
+    float v = 0.0f, w = 0.0f;
     if (threadIdx.x < 32) {
         const bool have = threadIdx.x < NT / 32;
-        float v = have ? warp_s[threadIdx.x] : 0.0f, w = have ? warp_c[threadIdx.x] : 0.0f;
+        v = have ? warp_s[threadIdx.x] : 0.0f;
+        w = have ? warp_c[threadIdx.x] : 0.0f;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
             const float ov = __shfl_xor_sync(0xffffffffu, v, off), ow = __shfl_xor_sync(0xffffffffu, w, off);
             w += ow;
             two_sum(v, w, ov);
         }
-        if (threadIdx.x == 0) *out = (v + w) * scale;
     }
+    return make_float2(v, w);
 }
 
 // *loss = scale * (sum of nblocks partials), by one whole block of NT
@@ -532,7 +541,8 @@ __device__ __forceinline__ void l1_final_block(const float* partial, long long n
 #pragma unroll
         for (int k = 0; k < 8; ++k) two_sum(s, c, v[k]);
     }
-    block_sum_pairs<NT>(s, c, scale, loss);
+    const float2 sum = block_sum_pairs<NT>(s, c);
+    if (threadIdx.x == 0) *loss = (sum.x + sum.y) * scale;
 }
 
 }  // namespace drp

@@ -12,14 +12,6 @@ namespace drp {
 constexpr int kLossThreads = 256;
 constexpr int kLossBlocksPerSM = 8;
 
-// Kahan step: s + x with the lost low part carried in c.
-__device__ inline void kahan_add(float& s, float& c, float x) {
-    const float y = x - c;
-    const float t = s + y;
-    c = (t - s) - y;
-    s = t;
-}
-
 __device__ inline float l1_grad(float d, float scale) { return d > 0.0f ? scale : (d < 0.0f ? -scale : 0.0f); }
 
 // Block sum of the threads' partial sums (block of kLossThreads).
