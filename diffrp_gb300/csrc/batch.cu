@@ -1790,7 +1790,7 @@ template <int TL, bool FIT>
 static void launch_batch_fine(const BatchArgs& a, cudaStream_t s) {
     switch (a.tpt) {
     case 0:
-        if (fine_many(TL, a.total_tiles)) launch_batch_fine<TL, 0, FIT, fine_threads_many<TL>()>(a, s);
+        if (fine_many(TL, a.total_tiles, a.total_prims)) launch_batch_fine<TL, 0, FIT, fine_threads_many<TL>()>(a, s);
         else launch_batch_fine<TL, 0, FIT>(a, s);
         break;
     case 1: launch_batch_fine<TL, 1, FIT>(a, s); break;

@@ -327,8 +327,9 @@ template <int TL>
 static void launch_fine(const RasterArgs& args, int tpt, cudaStream_t s) {
     constexpr int NT = fine_threads<TL>(), NM = fine_threads_many<TL>();
     dim3 grid((unsigned)(args.tiles_x * args.tiles_y), (unsigned)args.B);
-    // resident CTAs per SM of the instantiations (launch bounds: 4 above
-    // 8-pixel tiles); the fill cursors are spent by now and hold the order
+    // resident CTAs per SM of the instantiations that launch few tiles (launch
+    // bounds: 4 above 8-pixel tiles); the fill cursors are spent by now and hold
+    // the order
     const long long slots = (long long)drp_current_sm_count() * (TL == 3 ? 12 : 4);
     const long long ntiles = (long long)grid.x * grid.y;
     RasterArgs a = args;
@@ -339,7 +340,7 @@ static void launch_fine(const RasterArgs& args, int tpt, cudaStream_t s) {
     }
     switch (tpt) {
     case 0:
-        if (fine_many(TL, ntiles)) {
+        if (fine_many(TL, ntiles, a.max_view_tris * a.B)) {
             if (a.prev_key) fine_raster_kernel<TL, 0, true, NM><<<grid, NM, 0, s>>>(a);
             else fine_raster_kernel<TL, 0, false, NM><<<grid, NM, 0, s>>>(a);
         } else {

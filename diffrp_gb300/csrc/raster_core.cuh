@@ -473,16 +473,22 @@ struct FineTile {
 // tiles 285 against 214, 23,000 (ten meshes) 445 against 405, six views of
 // 800 x 1000 (18,900) 173 against 121.  32-pixel tiles have four times the list:
 // 3,375 tiles 224 against 235, 7,300 655 against 679, 16,384 (64 views of
-// 512 x 512) 300 against 244.
+// 512 x 512) 300 against 244.  Lists of large triangles that fill a pass of 256
+// take two or three of 128: from 64 triangles of the mesh per tile on, the rough
+// meshes lose more than the smooth ones gain (whole renders, four views of 1024 x
+// 1024, 16-pixel tiles: 78 per tile, rough 831 with 256 against 901 with 128,
+// smooth 398 against 378; 44 per tile 573 against 600 and 352 against 311; twelve
+// views, 32-pixel tiles: 589 per tile 3356 against 3906 and 1032 against 986).
 template <int TILE_LOG2>
 __host__ __device__ constexpr int fine_threads() { return TILE_LOG2 == 3 ? 64 : 256; }
 template <int TILE_LOG2>
 __host__ __device__ constexpr int fine_threads_many() { return TILE_LOG2 == 3 ? 64 : 128; }
 template <int TILE_LOG2, int NT>
 __host__ __device__ constexpr int fine_ctas() { return TILE_LOG2 == 3 ? 12 : 1024 / NT; }
-constexpr long long kFineManyTiles16 = 4864, kFineManyTiles32 = 12288;
-static inline bool fine_many(int tile_log2, long long tiles) {
-    return tile_log2 >= 4 && tiles >= (tile_log2 == 4 ? kFineManyTiles16 : kFineManyTiles32);
+constexpr long long kFineManyTiles16 = 4864, kFineManyTiles32 = 12288, kFineManyPrims = 64;
+static inline bool fine_many(int tile_log2, long long tiles, long long prims) {
+    return tile_log2 >= 4 && tiles >= (tile_log2 == 4 ? kFineManyTiles16 : kFineManyTiles32) &&
+           prims < kFineManyPrims * tiles;
 }
 
 // A list this long (pixel-parallel fine raster) has its small primitives
