@@ -9,6 +9,8 @@
 // of four.  The backward scatters attribute gradients with float4 atomics
 // after a warp-segmented reduction over runs of pixels that share a triangle, or,
 // in larger launches, by columns of pixels (walk.cuh).
+#include <algorithm>
+
 #include "drp_common.cuh"
 #include "drp_internal.h"
 #include "walk.cuh"
@@ -489,12 +491,19 @@ int launch_interp_fwd(const InterpArgs& a, cudaStream_t s) {
 // 700 x 700 38.6 / 33.5; 16 38.3 / 34.5; 1 at 4.2M 76.4 / 75.6 (2M 37.3 / 43.3).
 // 12 (a walk of eight and one of four) stays: 4.2M 155 / 170.  With derivatives:
 // 5 of 2 at 4.2M 194 / 165 (1M 52.6 / 53.7), 8 of 2 171 / 160, 4 of 4 134 / 143.
-static long long interp_walk_pixels(int C, bool da) {
+// Up to four channels or with derivatives a pixel costs the walk little more than
+// a triangle that the column leaves, so meshes of triangles of a few pixels stay
+// by pixels too (kWalkPixelsPerPrim; 318k triangles a view, six views of 800 x
+// 1000: 1 channel 86 by pixels against 115, 2 100 / 121, 4 100 / 119, 3 of 2
+// derivatives 148 / 176; 1440 x 1080, five pixels a triangle: 3 49 / 52).
+constexpr long long kWalkPixelsPerPrim = 6;
+static long long interp_walk_pixels(int C, bool da, long long prims) {
     const long long never = 1ll << 62;
     if (C % 8 == 4 && (C > 4 || da)) return never;
-    if (da) return C < 3 ? never : 1ll << 22;
-    if (C <= 2) return 1ll << 22;
-    return C == 4 ? 1ll << 21 : (C == 8 ? 1ll << 20 : 1ll << 19);
+    const long long few = C <= 4 || da ? kWalkPixelsPerPrim * prims : 0;
+    if (da) return C < 3 ? never : std::max(1ll << 22, few);
+    if (C <= 2) return std::max(1ll << 22, few);
+    return std::max(C == 4 ? 1ll << 21 : (C == 8 ? 1ll << 20 : 1ll << 19), few);
 }
 
 // Rows per warp: from 2^20 pixels on 16, for fewer sums to add (3 channels, a mesh
@@ -507,7 +516,7 @@ int launch_interp_bwd(const InterpArgs& a, cudaStream_t s) {
     if (n == 0) return 0;
     const bool da = a.nd > 0 && a.grad_da;
     const int rows = interp_walk_rows(a.C, n);
-    if (n < interp_walk_pixels(a.C, da))
+    if (n < interp_walk_pixels(a.C, da, a.num_triangles * a.B))
         interp_bwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a);
     else if (da)
         interp_bwd_walk_kernel<true><<<walk_blocks(a.B, a.H, a.W, rows), 32 * kWalkWarps, 0, s>>>(a, rows);
