@@ -414,8 +414,10 @@ static void launch_aa_setup(const AAArgs& a, cudaStream_t s) {
 // From this many pixels on the forward goes by regions.  Below, a warp's chain
 // of loads (ids, then records) is what counts: one 200 x 200 view of 3 channels
 // takes 21.3 us by regions of one row and 20.8 by pixels (forward and backward;
-// 27.6 and 26.2 with a mesh of 82k triangles), one of 512 x 512 22.8 and 25.0.
-constexpr long long kFwdRegionPixels = 1ll << 17;
+// 27.6 and 26.2 with a mesh of 82k triangles), one of 512 x 512 22.8 and 25.0.  The
+// forms cross between 400 x 400 (the whole call of an 82k mesh 47 us by pixels, 49
+// by regions) and 430 x 430 (50 and 48).
+constexpr long long kFwdRegionPixels = 11ll << 14;
 
 int launch_aa_fwd(const AAArgs& a, cudaStream_t s) {
     const int npix = a.H * a.W;
