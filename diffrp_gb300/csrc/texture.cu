@@ -551,9 +551,14 @@ __device__ __forceinline__ void bilin_bwd4(const Quad& q, float* glvl, const Bil
     gv = fmaf(dy, (float)h, gv);
 }
 
+// What a backward kernel is compiled for: each holds only its own path, whose
+// registers the others would take (nearest, 1 channel, 300 x 400 in the kernel
+// of the channel groups 10.0 us, before it had them 7.6, alone 8.3).
+constexpr int kTexBwdChannels = 0, kTexBwdQuad = 1, kTexBwdNearest = 2;
+
 // One pixel's gradients: texel gradients added into the levels, the uv and
 // uv_da gradients written.
-template <bool VEC4>
+template <int KIND>
 __device__ __forceinline__ void tex_bwd_pixel(const TexArgs& a, long long p, const TexIn& in) {
     const float u = in.u, v = in.v;
     const int n = (int)(p / a.view_pix), tn = a.Nt == 1 ? 0 : n;
@@ -561,7 +566,7 @@ __device__ __forceinline__ void tex_bwd_pixel(const TexArgs& a, long long p, con
     const float* g = a.grad_out + p * C;
     float gu = 0.f, gv = 0.f, gb = 0.f;
     float4 gda = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (a.filter == kTexNearest) {
+    if constexpr (KIND == kTexBwdNearest) {
         float* G0 = grad_level(a, 0, tn);
         const int i = nearest_index(a, u, v);
         const unsigned active = __activemask();
@@ -576,7 +581,7 @@ __device__ __forceinline__ void tex_bwd_pixel(const TexArgs& a, long long p, con
         const float f = L.f;
         const bool want_dl = (a.grad_uv_da || a.grad_bias) && L.interior;
         float dl = 0.f;  // d out / d lambda . grad_out
-        if constexpr (VEC4) {
+        if constexpr (KIND == kTexBwdQuad) {
             const float4 g4 = reinterpret_cast<const float4*>(a.grad_out)[p];
             const Quad q0 = fetch_quad(P0, B0);
             bilin_bwd4(q0, grad_level(a, L.l0, tn), B0, L.l0, tn, a.Nt > 1, a.lw[L.l0], a.lh[L.l0], g4,
@@ -647,7 +652,7 @@ __device__ __forceinline__ void tex_bwd_pixel(const TexArgs& a, long long p, con
 
 // kTexPix pixels per thread, blockDim.x apart (the warp's lanes take each
 // pixel together: its atomics are aggregated over the warp).
-template <bool VEC4>
+template <int KIND>
 __global__ void __launch_bounds__(256, 3) tex_bwd_kernel(TexArgs a) {
     const long long base = (long long)blockIdx.x * (kTexPix * blockDim.x) + threadIdx.x;
     TexIn in[kTexPix];
@@ -656,7 +661,7 @@ __global__ void __launch_bounds__(256, 3) tex_bwd_kernel(TexArgs a) {
         if (base + j * blockDim.x < a.npix) in[j] = tex_inputs(a, base + j * blockDim.x);
 #pragma unroll
     for (int j = 0; j < kTexPix; ++j)
-        if (base + j * blockDim.x < a.npix) tex_bwd_pixel<VEC4>(a, base + j * blockDim.x, in[j]);
+        if (base + j * blockDim.x < a.npix) tex_bwd_pixel<KIND>(a, base + j * blockDim.x, in[j]);
 }
 
 __device__ __forceinline__ float vadd(float a, float b) { return a + b; }
@@ -924,8 +929,9 @@ DRP_API int drp_texture_bwd(const float* tex, const float* pyr, int num_tex, int
     if (a.npix > 0) {
         const long long per_block = 256 * drp::kTexPix;
         const unsigned grid = (unsigned)((a.npix + per_block - 1) / per_block);
-        if (a.vec4) drp::tex_bwd_kernel<true><<<grid, 256, 0, s>>>(a);
-        else drp::tex_bwd_kernel<false><<<grid, 256, 0, s>>>(a);
+        if (a.filter == drp::kTexNearest) drp::tex_bwd_kernel<drp::kTexBwdNearest><<<grid, 256, 0, s>>>(a);
+        else if (a.vec4) drp::tex_bwd_kernel<drp::kTexBwdQuad><<<grid, 256, 0, s>>>(a);
+        else drp::tex_bwd_kernel<drp::kTexBwdChannels><<<grid, 256, 0, s>>>(a);
         drp_note_launch();
     }
     if (levels > 1 && a.filter >= drp::kTexMipNearest) {
