@@ -54,7 +54,7 @@ def _register():
         "drp_batch_block_maps": [P, I, P, P],
         "drp_batch_workspace_size": [LL, LL, ULL, ctypes.POINTER(ctypes.c_size_t)],
         "drp_batch_aa_state_size": [LL, ctypes.POINTER(ctypes.c_size_t)],
-        "drp_batch_fit_words_size": [LL, ctypes.POINTER(ctypes.c_size_t)],
+        "drp_batch_fit_words_size": [LL, LL, LL, ctypes.POINTER(ctypes.c_size_t)],
         "drp_batch_forward": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL, ctypes.c_uint,
                               P, P, P, P, LL, P],
         "drp_batch_render": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL, ctypes.c_uint,
@@ -265,17 +265,18 @@ class BatchRenderer:
         return out
 
     # -- execution -------------------------------------------------------------------
-    def _workspace(self, cap, fit=False):
+    def _workspace_bytes(self, cap, fit=False):
         """fit: with the pixel words of a gradient-forming forward."""
         nbytes = _ffi.size_out("drp_batch_workspace_size", self.total_prims, self.total_tiles, cap)
-        if fit:
-            nbytes += self._fit_words()
-        return self._wsh.get(nbytes, self.device)
+        return nbytes + self._fit_words() if fit else nbytes
+
+    def _workspace(self, cap):
+        return self._wsh.get(self._workspace_bytes(cap), self.device)
 
     def _fit_words(self):
         """Bytes of the pixel words: 0 where the gradient-forming forward takes
         the form for small launches, which fills the whole colour image."""
-        return _ffi.size_out("drp_batch_fit_words_size", self.total_pixels)
+        return _ffi.size_out("drp_batch_fit_words_size", self.total_pixels, self.image_floats, self.total_prims)
 
     def _blends_in_place(self):
         """Whether images for no backward take drp_batch_render, which writes one
@@ -343,7 +344,8 @@ class BatchRenderer:
         bufs = (rast.data_ptr(), None if color is None else color.data_ptr(), optr, fptr, npix)
         self._fwd_gen += 1
         fit = l1 is not None and len(l1) == 7
-        ws = self._workspace(cap, fit)
+        ws_bytes = self._workspace_bytes(cap, fit)
+        ws = self._wsh.get(ws_bytes, self.device)
         stream = _ffi.stream_of(self.device)
         args = (self._items_dev.data_ptr(), len(self.items), self._pmap.data_ptr(), self.prim_blocks,
                 self._xmap.data_ptr(), self.pixel_blocks, self.total_prims, self.total_tiles, pos.data_ptr(),
@@ -369,7 +371,7 @@ class BatchRenderer:
         else:
             tail = (stream,)
             entry = "drp_batch_forward"
-        _ffi.call(entry, ws.data_ptr(), ws.numel(), *args, cap, depth, *bufs, *tail)
+        _ffi.call(entry, ws.data_ptr(), ws_bytes, *args, cap, depth, *bufs, *tail)
         if first:
             # exact lists, sized synchronously; they also give the largest tile
             torch.cuda.current_stream(self.device).synchronize()

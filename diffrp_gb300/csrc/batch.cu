@@ -438,14 +438,11 @@ struct ItemGrad<true> {
     }
 };
 
-// Launches of at least this many pixels, with room in the workspace for the
-// pixel words, form the loss and its gradient with batch_fit_kernel, others with
-// batch_aa_l1_grad_kernel, whose shorter chain per pixel is what counts while the
-// regions fill only part of the chip: one view of 400 x 400 takes 58.5 with the
-// first against 55.3 us per step with the second at 3 channels and 68.2 against
-// 63.8 at 8; 724 x 724 84.2 against 88.6 and 81.2 against 84.0 (but 12 channels 6
-// percent more); from 1024 x 1024 on 3 to 8 and 16 channels are 7 to 40 percent
-// faster, 12 even.
+// Launches of at least this many pixels may form the loss and its gradient with
+// batch_fit_kernel (fit_words_bytes); the others take batch_aa_l1_grad_kernel, whose
+// shorter chain per pixel is what counts while the regions fill only part of the
+// chip: one view of 400 x 400 takes 58.5 with the first against 55.3 us per step with
+// the second at 3 channels and 68.2 against 63.8 at 8.
 constexpr long long kFitPixels = 1ll << 20;
 
 // batch_fit_kernel takes regions of 32 x 16 pixels, a fixed number per raster
@@ -1685,9 +1682,27 @@ static size_t aa_state_bytes(long long total_pixels, size_t* list_off) {
 }
 
 // Pixel words of batch_fit_kernel: they follow the workspace, whose size the
-// entries are told.
-static size_t fit_words_bytes(long long total_pixels) {
-    return total_pixels >= kFitPixels ? (size_t)total_pixels * 4 : 0;
+// entries are told; none where batch_aa_l1_grad_kernel is the faster.  Its time over
+// that kernel's per step, by channels, meshes of one triangle to 3, 13, 50, 800
+// pixels: one view of 1024 x 1024 1 .. 4 channels 1.15, 1.05, 1.0, 1.0 (3: 1.16, -,
+// 1.0, 0.9), 5 .. 8 1.15, 1.04, 0.9, 0.8; 1.3M pixels and more up to 8 channels 1.0,
+// 0.95, 0.9, 0.8 (rough meshes with a silhouette at most pixels 1.0 to 1.1 at 3
+// pixels a triangle).  More than 8 channels go row by row (fit_rows): the sums of
+// every row go out, whose atomics collide on few vertices (9 .. 11 channels, 800
+// pixels a triangle 1.1 to 1.35), and the four channels of 12, 20 or 28 past the
+// eights cost a pass of their own (one 1024 x 1024 view 1.1 to 1.2; from 2M pixels
+// 0.9 to 1.0, 12 on a coarse mesh 1.2).
+static size_t fit_words_bytes(long long pixels, long long image_floats, long long prims) {
+    if (pixels < kFitPixels) return 0;
+    const long long C = (image_floats + pixels - 1) / pixels;
+    bool fit;
+    if (C <= 8)
+        fit = pixels >= 5ll << 18 || ((C == 3 || C >= 5) && prims <= pixels / 16);
+    else if (C % 4 == 0 && C >= 16)
+        fit = pixels >= (C % 8 == 0 ? 3ll << 19 : 1ll << 21);
+    else
+        fit = pixels >= (C == 12 ? 1ll << 21 : 3ll << 19) && prims >= pixels / 256;
+    return fit ? (size_t)pixels * 4 : 0;
 }
 
 static void carve_aa_state(BatchArgs& a, void* state, long long total_pixels) {
@@ -2049,9 +2064,11 @@ DRP_API int drp_batch_aa_state_size(long long total_pixels, size_t* bytes) {
     return DRP_STATUS_OK;
 }
 
-DRP_API int drp_batch_fit_words_size(long long total_pixels, size_t* bytes) {
-    if (!bytes || total_pixels <= 0) return bfail("drp_batch_fit_words_size: bad arguments");
-    *bytes = drp::fit_words_bytes(total_pixels);
+DRP_API int drp_batch_fit_words_size(long long total_pixels, long long image_floats, long long total_prims,
+                                     size_t* bytes) {
+    if (!bytes || total_pixels <= 0 || image_floats < total_pixels || total_prims < 0)
+        return bfail("drp_batch_fit_words_size: bad arguments");
+    *bytes = drp::fit_words_bytes(total_pixels, image_floats, total_prims);
     return DRP_STATUS_OK;
 }
 
@@ -2241,8 +2258,8 @@ static int batch_fit_l1(const char* who, bool full_color, void* workspace, size_
     a.color = color;
     a.out = out;
     carve_aa_state(a, aa_state, total_pixels);
-    const size_t words = drp::fit_words_bytes(total_pixels);
-    a.fit = words > 0 && workspace_bytes >= L.total + words;
+    // room for the pixel words chooses the form (fit_words_bytes)
+    a.fit = total_pixels >= drp::kFitPixels && workspace_bytes >= L.total + (size_t)total_pixels * 4;
     a.aa_words = a.fit ? reinterpret_cast<uint32_t*>(static_cast<char*>(workspace) + L.total) : nullptr;
     a.emit_color = full_color;  // else the loss pass stores the listed pixels' colours only
     a.emit_out = false;  // the fused antialias + loss pass writes every output pixel

@@ -445,12 +445,14 @@ int drp_batch_render(void* workspace, size_t workspace_bytes, const drp_batch_it
 int drp_batch_aa_state_size(long long total_pixels, size_t* bytes);
 
 /*
- * Bytes that the large-launch form of drp_batch_fit_l1 / drp_batch_forward_l1_grad
- * uses of the workspace after drp_batch_workspace_size bytes: 0 below 2^20
- * pixels, where there is no such form.  With a smaller workspace those entries
- * take the form for small launches.
+ * Bytes to add to drp_batch_workspace_size for drp_batch_fit_l1 /
+ * drp_batch_forward_l1_grad, whose large-launch form keeps a word per pixel there:
+ * 0 where the form for small launches is the faster (below 2^20 pixels there is
+ * no other).  image_floats, total_prims: totals[3] and [0] of drp_batch_plan.  The
+ * entries take the large-launch form when workspace_bytes has room for the words,
+ * so pass the sum of the two queries, not the size of a larger buffer.
  */
-int drp_batch_fit_words_size(long long total_pixels, size_t* bytes);
+int drp_batch_fit_words_size(long long total_pixels, long long image_floats, long long total_prims, size_t* bytes);
 
 /*
  * drp_batch_forward with the mean-absolute-error loss against target (image

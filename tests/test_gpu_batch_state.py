@@ -27,9 +27,8 @@ def test_state_size_is_the_layout_of_this_abi_version():
 @pytest.mark.parametrize("sizes", [[(70, 90), (33, 20)], [(1000, 1101), (33, 20)]])
 def test_nothing_is_written_past_the_state(cuda_lib, monkeypatch, entry, sizes):
     r, pos, attr, target = _renderer(sizes, (4, 7), 4)
-    plain = r._workspace
     if entry == "fit_l1_plain_workspace":
-        monkeypatch.setattr(r, "_workspace", lambda cap, fit=False: plain(cap))
+        monkeypatch.setattr(r, "_fit_words", lambda: 0)
     n, scale = _state_bytes(r.total_pixels), 1.0 / r.image_floats
     state = torch.full((n + 8 * r.total_pixels,), 0xA5, dtype=torch.uint8, device="cuda")
     rast, col = r._buffers()
@@ -48,10 +47,12 @@ def test_nothing_is_written_past_the_state(cuda_lib, monkeypatch, entry, sizes):
     r._forward_raw(pos, attr.reshape(-1), rast, col, img, l1, flags=state)
     assert int(state[:4].view(torch.int32)) > 0  # listed pixels
     assert bool((state[n:] == 0xA5).all())
+    whole = entry != "fit_l1" or r._fit_words() == 0
+    assert whole == (entry != "fit_l1" or r.total_pixels < 1 << 20)
     monkeypatch.undo()
     _, color, out = r.forward_buffers(pos, attr)
     assert torch.equal(img, out)
-    if entry != "fit_l1" or r.total_pixels < 1 << 20:
+    if whole:
         assert torch.equal(col, color)
     if l1 is not None and len(l1) == 7:
         p, a = pos.clone().requires_grad_(True), attr.clone().requires_grad_(True)

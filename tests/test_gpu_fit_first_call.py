@@ -13,8 +13,10 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("recompute", [False, True])
 @pytest.mark.parametrize("tile_log2,hw", [(3, (401, 390)), (4, (1040, 1030))])  # per-pixel and region form
-def test_first_call_with_overflowing_lists(cuda_lib, recompute, tile_log2, hw):
+def test_first_call_with_overflowing_lists(cuda_lib, monkeypatch, recompute, tile_log2, hw):
     from diffrp_gb300.batch import BatchRenderer
+    monkeypatch.setattr(BatchRenderer, "_fit_words",
+                        lambda self: 4 * self.total_pixels if self.total_pixels >= 1 << 20 else 0)
     v, f = S.icosphere(1, 0.8)
     rng = np.random.default_rng(0)
     pos = []

@@ -10,6 +10,12 @@ pytestmark = pytest.mark.gpu
 HW = 1024
 
 
+@pytest.fixture(autouse=True)
+def region_form(monkeypatch):
+    from diffrp_gb300.batch import BatchRenderer
+    monkeypatch.setattr(BatchRenderer, "_fit_words", lambda self: 4 * self.total_pixels)
+
+
 def _loss(views, C, fill):
     from diffrp_gb300.batch import BatchRenderer
     v, f = S.icosphere(1, 0.8)
