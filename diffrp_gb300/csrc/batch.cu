@@ -417,9 +417,10 @@ __device__ __forceinline__ int find_item_by_pixel(const drp_batch_item* items, i
 // sum d/du, d/dv by shuffles.  Grid-stride over the device-side count, so
 // the launch needs no host sync; the grid is one resident wave
 // (list_kernel_grid).  L1G (the forward that forms the loss's gradient): the
-// kernel follows the antialias / loss pass on the launch chain, and its last
-// block first adds the loss from that pass's partials (no separate
-// final-sum launch).
+// kernel follows the antialias / loss pass on the launch chain and forms the
+// loss before its pixels, without a separate final-sum launch: its last block
+// from batch_aa_l1_grad_kernel's partials, or every block a slice of
+// batch_fit_kernel's region sums (fit_loss).
 // The incoming image gradient of one item: the gradient buffer times the
 // upstream scale, or (L1G, the forward that forms the loss's gradient) the
 // L1 sign gradient from the output and the target.
@@ -864,7 +865,7 @@ __device__ __forceinline__ void store4(float* p, int n, const float (&x)[4]) {
 }
 
 // Antialias + L1 loss with the loss's gradient formed in the same pass, for
-// launches of at least kFitPixels (drp_batch_fit_l1,
+// large launches (fit_words_bytes; drp_batch_fit_l1,
 // drp_batch_forward_l1_grad).  Every pixel: its colour, interpolated again
 // from its rast row (the attribute rows are needed for the backward anyway, so
 // no colour image is written and read back), the blend, the output and the
@@ -1557,8 +1558,9 @@ __device__ __forceinline__ void pixel_backward_l1(const BatchArgs& a, const drp_
 }
 
 // Antialias + L1 loss with the loss's gradient formed in the same pass, one
-// thread per pixel, from a stored colour image: the form for launches below
-// kFitPixels (batch_fit_kernel above).  Every pixel: its output and |error| partial
+// thread per pixel, from a stored colour image: the form for the launches that
+// batch_fit_kernel does not take (fit_words_bytes).  Every pixel: its output and
+// |error| partial
 // as batch_aa_l1_kernel computes them.  Then, for the pixels no blending pair
 // touches (the listed ones belong to batch_aa_bwd_kernel, which forms
 // the sign from the output and the target), the pixel's whole backward with
@@ -1921,8 +1923,8 @@ int launch_batch_forward(BatchArgs a, void* ws, const BatchLayout& L, cudaStream
                 launch_pdl(batch_aa_l1_grad_kernel, dim3((unsigned)a.n_pix_blocks), dim3(256), s, a);
             }
             drp_note_launch();
-            // the listed pixels' whole backward, and (its last block) the
-            // final loss sum: one launch on the chain
+            // the listed pixels' whole backward, and the final loss sum
+            // (the last block's, or fit_loss by all): one launch on the chain
             if (a.fit)
                 launch_pdl(batch_aa_bwd_kernel<kListFit, kListLanes>,
                            dim3((unsigned)list_kernel_grid<kListFit>(a.n_pix_blocks)), dim3(256), s, a);
@@ -2224,8 +2226,8 @@ DRP_API int drp_batch_forward_l1(void* workspace, size_t workspace_bytes, const 
     return drp_check_launch("drp_batch_forward_l1");
 }
 
-static int batch_fit_l1(const char* who, bool full_color, void* workspace, size_t workspace_bytes, const drp_batch_item* items,
-                        int num_items, const int* prim_block_map, long long prim_blocks,
+static int batch_fit_l1(const char* who, bool full_color, void* workspace, size_t workspace_bytes,
+                        const drp_batch_item* items, int num_items, const int* prim_block_map, long long prim_blocks,
                         const int* pixel_block_map, long long pixel_blocks, long long total_prims,
                         long long total_tiles, const float* pos, const int* tri, const float* attr,
                         const int* nbr, int tile_log2, int threads_per_tri,
@@ -2289,10 +2291,11 @@ DRP_API int drp_batch_forward_l1_grad(void* workspace, size_t workspace_bytes, c
                                       float* out, void* aa_state, long long total_pixels, const float* target,
                                       float scale, float* block_loss, float* loss, float* grad_pos, float* grad_attr,
                                       float* zero_first, long long zero_floats, void* stream) {
-    return batch_fit_l1("drp_batch_forward_l1_grad", true, workspace, workspace_bytes, items, num_items, prim_block_map, prim_blocks, pixel_block_map, pixel_blocks,
-                       total_prims, total_tiles, pos, tri, attr, nbr, tile_log2, threads_per_tri, list_capacity, bin_depth,
-                       rast, color, out, aa_state, total_pixels, target, scale, block_loss, loss, grad_pos, grad_attr,
-                       zero_first, zero_floats, stream);
+    return batch_fit_l1("drp_batch_forward_l1_grad", true, workspace, workspace_bytes, items, num_items,
+                        prim_block_map, prim_blocks, pixel_block_map, pixel_blocks, total_prims, total_tiles, pos, tri,
+                        attr, nbr, tile_log2, threads_per_tri, list_capacity, bin_depth, rast, color, out, aa_state,
+                        total_pixels, target, scale, block_loss, loss, grad_pos, grad_attr, zero_first, zero_floats,
+                        stream);
 }
 
 DRP_API int drp_batch_fit_l1(void* workspace, size_t workspace_bytes, const drp_batch_item* items,
@@ -2304,10 +2307,11 @@ DRP_API int drp_batch_fit_l1(void* workspace, size_t workspace_bytes, const drp_
                              float* out, void* aa_state, long long total_pixels, const float* target,
                              float scale, float* block_loss, float* loss, float* grad_pos, float* grad_attr,
                              float* zero_first, long long zero_floats, void* stream) {
-    return batch_fit_l1("drp_batch_fit_l1", false, workspace, workspace_bytes, items, num_items, prim_block_map, prim_blocks, pixel_block_map, pixel_blocks,
-                       total_prims, total_tiles, pos, tri, attr, nbr, tile_log2, threads_per_tri, list_capacity, bin_depth,
-                       rast, color, out, aa_state, total_pixels, target, scale, block_loss, loss, grad_pos, grad_attr,
-                       zero_first, zero_floats, stream);
+    return batch_fit_l1("drp_batch_fit_l1", false, workspace, workspace_bytes, items, num_items, prim_block_map,
+                        prim_blocks, pixel_block_map, pixel_blocks, total_prims, total_tiles, pos, tri, attr, nbr,
+                        tile_log2, threads_per_tri, list_capacity, bin_depth, rast, color, out, aa_state,
+                        total_pixels, target, scale, block_loss, loss, grad_pos, grad_attr, zero_first, zero_floats,
+                        stream);
 }
 
 DRP_API int drp_batch_colors(const drp_batch_item* items, int num_items, const int* pixel_block_map,
