@@ -81,19 +81,27 @@ class _SharedWorkspace:
     """The batch workspace buffer, shared by a renderer and its recompute
     chunks (one buffer sized for the largest user).  records = (buffer,
     renderer id, forward generation) of the forward whose antialias records
-    the buffer holds."""
+    the buffer holds.  A buffer that grows is replaced: given back when only the
+    stream it was allocated on has used it, else kept (retired), for the CUDA
+    graphs captured on it and the work other streams may still have on it."""
 
     def __init__(self):
         self.buf = None
-        self.retired = []  # replaced buffers, kept alive for CUDA graphs captured on them
+        self.stream = None   # of the buffer's allocation
+        self.kept = False    # captured, or used on another stream
+        self.retired = []
         self.records = None
 
     def get(self, nbytes, device):
+        stream = _ffi.stream_of(device)
         if self.buf is None or self.buf.numel() < nbytes:
-            if self.buf is not None:
+            if self.kept:
                 self.retired.append(self.buf)
+            self.buf = self.records = None
             self.buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
-            self.records = None
+            self.stream, self.kept = stream, False
+        if stream != self.stream or torch.cuda.is_current_stream_capturing():
+            self.kept = True
         return self.buf
 
 
