@@ -54,7 +54,7 @@ def _register():
         "drp_batch_block_maps": [P, I, P, P],
         "drp_batch_workspace_size": [LL, LL, ULL, ctypes.POINTER(ctypes.c_size_t)],
         "drp_batch_aa_state_size": [LL, ctypes.POINTER(ctypes.c_size_t)],
-        "drp_batch_fit_words_size": [LL, LL, LL, ctypes.POINTER(ctypes.c_size_t)],
+        "drp_batch_fit_words_size": [LL, LL, LL, I, ctypes.POINTER(ctypes.c_size_t)],
         "drp_batch_forward": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL, ctypes.c_uint,
                               P, P, P, P, LL, P],
         "drp_batch_render": [P, ctypes.c_size_t, P, I, P, LL, P, LL, LL, LL, P, P, P, P, I, I, ULL, ctypes.c_uint,
@@ -284,7 +284,8 @@ class BatchRenderer:
     def _fit_words(self):
         """Bytes of the pixel words: 0 where the gradient-forming forward takes
         the form for small launches, which fills the whole colour image."""
-        return _ffi.size_out("drp_batch_fit_words_size", self.total_pixels, self.image_floats, self.total_prims)
+        return _ffi.size_out("drp_batch_fit_words_size", self.total_pixels, self.image_floats, self.total_prims,
+                             self.tile_log2)
 
     def _blends_in_place(self):
         """Whether images for no backward take drp_batch_render, which writes one

@@ -1684,26 +1684,53 @@ static size_t aa_state_bytes(long long total_pixels, size_t* list_off) {
 }
 
 // Pixel words of batch_fit_kernel: they follow the workspace, whose size the
-// entries are told; none where batch_aa_l1_grad_kernel is the faster.  Its time over
-// that kernel's per step, by channels, meshes of one triangle to 3, 13, 50, 800
-// pixels: one view of 1024 x 1024 1 .. 4 channels 1.15, 1.05, 1.0, 1.0 (3: 1.16, -,
-// 1.0, 0.9), 5 .. 8 1.15, 1.04, 0.9, 0.8; 1.3M pixels and more up to 8 channels 1.0,
-// 0.95, 0.9, 0.8 (rough meshes with a silhouette at most pixels 1.0 to 1.1 at 3
-// pixels a triangle).  More than 8 channels go row by row (fit_rows): the sums of
-// every row go out, whose atomics collide on few vertices (9 .. 11 channels, 800
-// pixels a triangle 1.1 to 1.35), and the four channels of 12, 20 or 28 past the
-// eights cost a pass of their own (one 1024 x 1024 view 1.1 to 1.2; from 2M pixels
-// 0.9 to 1.0, 12 on a coarse mesh 1.2).
-static size_t fit_words_bytes(long long pixels, long long image_floats, long long prims) {
+// entries are told; none where batch_aa_l1_grad_kernel's step is the faster.  A
+// region is half a 32-pixel tile, but two 16-pixel or eight 8-pixel ones, whose other
+// CTAs come and go for nothing; a walk pays by the pixels its columns stay in a
+// triangle; more than eight channels go row by row (fit_rows), whose sums collide on
+// few vertices (a plain multiple of eight has the fewest passes, four more than that a
+// pass of their own).  Step over the other form's, smooth meshes of 24, 10, 3 and 1
+// pixels a triangle and a coarse one (1280 triangles):
+//   32-pixel tiles, 1.0M pixels:  1 channel 1.01 1.06 1.09 1.05 0.96, 4 0.95 1.01 1.03
+//     1.03 0.92, 8 0.91 0.96 0.97 1.00 0.85, 9 0.86 0.92 0.88 0.92 1.13, 12 1.06 1.07
+//     1.05 1.02 1.13, 20 1.00 1.01 0.96 0.97 1.02, 32 0.8
+//   and 2.4M:  1 0.94 1.00 0.99 1.00 0.84, 4 0.9, 8 0.9, 9 0.8 (coarse 1.04), 12 1.0;
+//     8.4M and 24 pixels a triangle: 0.7 to 0.9
+//   16-pixel tiles, 1.0M:  1 1.10 1.15 1.17 1.17, 4 1.01 1.06 1.11 1.10, 8 1.02 1.07 1.09
+//     1.07 0.91, 12 1.2, 16 1.1;  1.7M:  1 1.03 1.06 1.11 1.10 0.84, 4 0.97 1.00 1.03
+//     1.05 0.86, 8 0.93 0.98 1.00 1.03 0.82, 13 0.8 (coarse 1.2), 12 1.1, 16 1.04;
+//     4.2M:  4 0.93 0.96 0.98 0.99, 12 1.05, 16 0.95
+//   8-pixel tiles, 4.2M:  1 1.1, 4 1.01 1.06 1.03 1.03, 8 0.98 1.04 1.02, 13 0.83, 12 1.1
+// (Rough meshes, a silhouette at most pixels, up to 0.1 more.)
+static size_t fit_words_bytes(long long pixels, long long image_floats, long long prims, int tile_log2) {
+    constexpr long long kMi = 1ll << 20, kNever = 1ll << 62;
     if (pixels < kFitPixels) return 0;
     const long long C = (image_floats + pixels - 1) / pixels;
-    bool fit;
-    if (C <= 8)
-        fit = pixels >= 5ll << 18 || ((C == 3 || C >= 5) && prims <= pixels / 16);
-    else if (C % 4 == 0 && C >= 16)
-        fit = pixels >= (C % 8 == 0 ? 3ll << 19 : 1ll << 21);
-    else
-        fit = pixels >= (C == 12 ? 1ll << 21 : 3ll << 19) && prims >= pixels / 256;
+    long long from = kNever, per_prim = 0;  // pixels of the launch, pixels per triangle
+    bool coarse = true;                     // also with more than 256 pixels per triangle
+    if (C <= 8) {
+        if (tile_log2 == 5) {
+            from = kMi;
+            if (C <= 2) per_prim = 2 * pixels < 3 * kMi ? 32 : (pixels < 2 * kMi ? 16 : 0);
+            else if (C <= 5) per_prim = 4 * pixels < 5 * kMi ? 12 : 0;
+        } else if (tile_log2 == 4) {
+            const bool few = 4 * pixels < 5 * kMi;
+            from = !few || C == 3 || C >= 5 ? kMi : kNever;
+            per_prim = few ? (C == 3 ? 64 : 32) : (C <= 2 ? 48 : (C <= 5 ? 16 : 4));
+        } else if (C >= 3) {
+            from = 4 * kMi;
+            per_prim = C <= 5 ? 48 : 16;
+        }
+    } else if (C % 8 == 0) {
+        if (tile_log2 == 5 || C >= 32) from = kMi;
+        else if (tile_log2 == 4) from = C >= 24 ? 3 * kMi / 2 : 2 * kMi;
+    } else {
+        coarse = false;
+        if (tile_log2 == 5) from = C == 12 ? 2 * kMi : (C % 4 == 0 ? 5 * kMi / 4 : kMi);
+        else if (C % 4 != 0) from = tile_log2 == 4 ? 5 * kMi / 4 : 4 * kMi;
+        else if (tile_log2 == 4 && C > 12) from = 2 * kMi;
+    }
+    const bool fit = pixels >= from && per_prim * prims <= pixels && (coarse || 256 * prims >= pixels);
     return fit ? (size_t)pixels * 4 : 0;
 }
 
@@ -2067,10 +2094,11 @@ DRP_API int drp_batch_aa_state_size(long long total_pixels, size_t* bytes) {
 }
 
 DRP_API int drp_batch_fit_words_size(long long total_pixels, long long image_floats, long long total_prims,
-                                     size_t* bytes) {
-    if (!bytes || total_pixels <= 0 || image_floats < total_pixels || total_prims < 0)
+                                     int tile_log2, size_t* bytes) {
+    if (!bytes || total_pixels <= 0 || image_floats < total_pixels || total_prims < 0 || tile_log2 < 3 ||
+        tile_log2 > 5)
         return bfail("drp_batch_fit_words_size: bad arguments");
-    *bytes = drp::fit_words_bytes(total_pixels, image_floats, total_prims);
+    *bytes = drp::fit_words_bytes(total_pixels, image_floats, total_prims, tile_log2);
     return DRP_STATUS_OK;
 }
 

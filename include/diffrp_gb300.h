@@ -452,7 +452,8 @@ int drp_batch_aa_state_size(long long total_pixels, size_t* bytes);
  * entries take the large-launch form when workspace_bytes has room for the words,
  * so pass the sum of the two queries, not the size of a larger buffer.
  */
-int drp_batch_fit_words_size(long long total_pixels, long long image_floats, long long total_prims, size_t* bytes);
+int drp_batch_fit_words_size(long long total_pixels, long long image_floats, long long total_prims, int tile_log2,
+                             size_t* bytes);
 
 /*
  * drp_batch_forward with the mean-absolute-error loss against target (image

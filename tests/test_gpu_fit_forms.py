@@ -1,24 +1,35 @@
 """The two forms of the gradient-forming forward: the rule that chooses between them
-by pixels, channels and triangles, and the large launch's form at the sizes and
+by tile, pixels, channels and triangles, and the large launch's form at the sizes and
 channel counts that the rule keeps from it."""
 import pytest
 
 from tests import test_gpu_fit as T
 
 
-@pytest.mark.parametrize("pixels,channels,prims,large", [
-    ((1 << 20) - 1, 8, 1000, False), (1 << 20, 8, 1000, True), (1 << 20, 8, (1 << 16) + 1, False),
-    (1 << 20, 4, 1000, False), (1 << 20, 3, 1000, True), ((5 << 18) - 1, 1, 1000, False), (5 << 18, 1, 1 << 20, True),
-    ((3 << 19) - 1, 16, 1000, False), (3 << 19, 16, 1000, True), (3 << 19, 32, 1000, True),
-    (3 << 19, 20, 1000, False), (1 << 21, 20, 1000, True),
-    (3 << 19, 9, 6143, False), (3 << 19, 9, 6144, True), ((3 << 19) - 1, 13, 1 << 20, False),
-    (3 << 19, 12, 1 << 20, False), (1 << 21, 12, 1 << 20, True), (1 << 23, 12, 1000, False)])
-def test_rule(pixels, channels, prims, large):
+MI = 1 << 20
+
+
+@pytest.mark.parametrize("tile,pixels,channels,prims,large", [
+    # up to eight channels: pixels and pixels per triangle by tile
+    (5, MI - 1, 8, 1000, False), (5, MI, 8, 2 * MI, True), (5, MI, 1, MI // 32, True), (5, MI, 1, MI // 32 + 1, False),
+    (5, 2 * MI, 1, 2 * MI, True), (5, MI, 4, MI // 12, True), (5, MI, 5, MI // 12 + 1, False),
+    (5, 5 * MI // 4, 5, MI, True), (4, MI, 4, 1, False), (4, MI, 3, MI // 64, True), (4, MI, 8, MI // 32 + 1, False),
+    (4, 5 * MI // 4 - 1, 2, 1, False), (4, 3 * MI // 2, 2, MI // 32, True), (4, 3 * MI // 2, 2, MI // 32 + 1, False),
+    (4, 2 * MI, 4, MI // 8, True), (4, 2 * MI, 5, MI // 8 + 1, False), (4, 2 * MI, 8, MI // 2, True),
+    (3, 8 * MI, 2, 1, False), (3, 4 * MI, 4, MI // 16, True), (3, 4 * MI, 8, MI // 4, True),
+    (3, 4 * MI - 1, 8, 1, False),
+    # more: multiples of eight, then the others, which a coarse mesh keeps out
+    (5, MI, 16, 1, True), (4, 2 * MI - 1, 16, 1, False), (4, 2 * MI, 16, 1, True), (4, 3 * MI // 2, 24, 1, True),
+    (3, MI, 32, 1, True), (3, 8 * MI, 16, 1, False),
+    (5, MI, 9, MI // 256, True), (5, MI, 9, MI // 256 - 1, False), (4, 5 * MI // 4, 13, MI, True),
+    (5, 2 * MI - 1, 12, MI, False), (5, 2 * MI, 12, MI, True), (4, 8 * MI, 12, MI, False),
+    (5, 5 * MI // 4, 20, MI, True), (4, 2 * MI, 20, MI, True), (3, 8 * MI, 20, MI, False), (3, 4 * MI, 13, MI, True)])
+def test_rule(tile, pixels, channels, prims, large):
     from diffrp_gb300 import _ffi, batch, build
     build.build()
     batch._register()
-    words = _ffi.size_out("drp_batch_fit_words_size", pixels, pixels * channels - 1 if channels > 1 else pixels, prims)
-    assert words == (4 * pixels if large else 0)
+    floats = pixels * channels - 1 if channels > 1 else pixels  # items of fewer channels among them
+    assert _ffi.size_out("drp_batch_fit_words_size", pixels, floats, prims, tile) == (4 * pixels if large else 0)
 
 
 @pytest.mark.gpu
@@ -29,6 +40,7 @@ def test_rule(pixels, channels, prims, large):
     (5, [(1060, 1020), (1040, 1030)], (9, 13), True, False),
     (4, [(1300, 1301)], (20, 20), False, True),
     (3, [(1030, 1033)], (16, 16), False, False),
+    (3, [(900, 601), (850, 700)], (8, 5), False, False),
     (4, [(400, 400)] * 17, (12, 10), False, False),  # walks of eight rows
 ])
 def test_either_form(cuda_lib, monkeypatch, large, tile_log2, sizes, channels, recompute, use_images):
